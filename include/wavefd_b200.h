@@ -471,11 +471,8 @@ int WFD_Codec_Gradient(void *codec, const float *blocks, long n, float *grad, fl
  * AdjointBornAccumulation_wavefieldsep / _wavefieldsep_V) for callers that cannot call cudaMalloc:
  * it allocates no memory. Every array must already be device or managed memory (nx*ny*nz floats,
  * z fastest; ny = 1 for 2D; wavefieldDM and mOld both NULL for the isotropic case); dVel is
- * accumulated. Its FFT scratch is a fixed 160 KiB device array inside the library, so nz is
- * limited to 2048 (larger nz returns WFD_ERR_ARG). The first call on each device looks up that
- * array's device address; make that first call before any stream capture, and do not use the
- * entry point across a cudaDeviceReset. The image must be on the current device. All calls share
- * the array (it keeps the tables of the last FFT length): calls that overlap on the GPU race. The
+ * accumulated. nz is limited to 2048 (larger nz returns WFD_ERR_ARG). The image must be on the
+ * current device. Calls on different streams are independent. The
  * arithmetic is the fast build's, or the bitwise-parity build's when WAVEFD_B200_STRICT=1 (as for
  * new propagator objects). Work is enqueued on `stream` (a cudaStream_t, NULL for the default
  * stream) without host synchronisation. Returns a WFD_* status. */

@@ -88,7 +88,6 @@ struct K {
     WFD_DISPATCH(born_aniso_v)
     WFD_DISPATCH(image_iso_v)
     WFD_DISPATCH(image_aniso_v)
-    WFD_DISPATCH(image_wavefieldsep)
     WFD_DISPATCH(born_iso_fused)
     WFD_DISPATCH(image_iso_fused)
     WFD_DISPATCH(born_vea_fused)
@@ -143,16 +142,10 @@ int prop_image(Prop *p, const char *variant, float *const *args, int nargs, long
     float **t = p->tmp;
     std::vector<float *> outs;
     if (!strncmp(variant, "wavefieldsep", 12)) {
-        const long ncols = g.nx * g.ny;
-        const long nfft = 2 * g.nz;
-        if (!p->work) {
-            long cols = ncols < 4096 ? ncols : 4096;
-            if (wfd::dMalloc(&p->work, sizeof(float2) * (size_t)cols * (size_t)nfft * 2) != cudaSuccess)
-                return prop_fail(p, WFD_ERR_ALLOC, "FFT workspace allocation failed");
-            p->work_cols = cols;
-        }
         float *dm = p->phys == ISO ? nullptr : a[2];
-        k.image_wavefieldsep(g, isfwi, F, a[1], (const float *)dm, a[0], p->work, p->work_cols, p->stream);
+        const bool ok = p->strict ? wfd_strict::image_wavefieldsep(g, isfwi, F, a[1], dm, a[0], p->stream)
+                                  : wfd_fast::image_wavefieldsep(g, isfwi, F, a[1], dm, a[0], p->stream);
+        if (!ok) return prop_fail(p, WFD_ERR_CUDA, "AdjointBornAccumulation: wavefield separation of columns this deep");
         outs.push_back(a[0]);
     } else if (p->phys == ISO) {
         if (!strcmp(variant, "V")) {

@@ -161,12 +161,9 @@ struct TileInfo {
     void image_vea_fused(const wfd::Grid &g, bool rot, const wfd::Fields &F, const float *dp,            \
                          const float *dm, const float *P, const float *M, float *dv, float *de, float *da, \
                          cudaStream_t s);                                                                \
-    void image_wavefieldsep(const wfd::Grid &g, long isfwi, const wfd::Fields &F, const float *dp,       \
-                            const float *dm, float *dv, float2 *work, long ncols_per_pass,               \
-                            cudaStream_t s);                                                             \
-    void image_wavefieldsep_tables(const wfd::Grid &g, long isfwi, const wfd::Fields &F, const float *dp, \
-                                   const float *dm, float *dv, const float2 *tables, int m,              \
-                                   cudaStream_t s);                                                      \
+    /* false: the column is too deep (nz > 8192) or the kernel cannot run */                             \
+    bool image_wavefieldsep(const wfd::Grid &g, long isfwi, const wfd::Fields &F, const float *dp,       \
+                            const float *dm, float *dv, cudaStream_t s);                                 \
     }
 
 WFD_DECLARE_LAUNCHERS(wfd_fast)

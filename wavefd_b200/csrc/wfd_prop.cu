@@ -224,7 +224,6 @@ void prop_destroy(Prop *p) {
         if (p->tmp[i]) cudaFree(p->tmp[i]);
     for (int i = 0; i < 7; i++)
         if (p->stage[i]) cudaFree(p->stage[i]);
-    if (p->work) cudaFree(p->work);
     if (p->own_stream && p->stream) cudaStreamDestroy(p->stream);
     delete p;
 }

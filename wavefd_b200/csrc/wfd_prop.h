@@ -33,9 +33,7 @@ struct Prop {
     float *field[F_COUNT] = {};
     float *tmp[12] = {};     // scratch of the unfused passes (the reference's tmp arrays)
     float *stage[7] = {};    // device copies of host arrays given to Born/imaging calls (first use)
-    float2 *work = nullptr;  // FFT workspace of the wavefield-separation condition
     float *illum = nullptr;  // caller's source illumination sum (device), accumulated by every step
-    long work_cols = 0;
     int status = WFD_OK;
     std::string message;
     long steps = 0;

@@ -2,246 +2,438 @@
 // prop3DAcoVTIDenQ_DEO2_FDTD.h:606-725; TTI prop3DAcoTTIDenQ_DEO2_FDTD.h:609-728; 2D Iso
 // prop2DAcoIsoDenQ_DEO2_FDTD.h:584-672), with a hand-written batched column FFT.
 //
-// Per (x,y) column and per field: zero-pad the column to nfft = 2nz, scale by 1/nfft,
-// transform with sign +1 (FFTW's "forward" here is +1), zero bins [n/2+1, n) of the forward
-// field and [kadj+1, kadj+n/2) of the adjoint field (kadj = 0 FWI, n/2 RTM), transform back
-// with sign -1, and accumulate 2B/V^3 * Re(a*b). One CTA per column, everything in shared
-// memory: radix-2 when nfft is a power of two, Bluestein's chirp-z convolution otherwise.
-#include <math.h>
-
-#include <vector>
-
+// The reference, per (x,y) column and per field: zero-pad the column to n = 2nz, transform, zero half
+// of the bins, transform back, and accumulate 2B/V^3 * Re(a*b), where a keeps bins 0..nz of the
+// forward field and b bins 0..nz (RTM) or 0 and nz..n-1 (FWI) of the adjoint field. Summing the kept
+// bins in closed form (only the first nz inputs are nonzero and only the first nz outputs are used)
+// leaves, for a column x,
+//   Re a_j = x_j / 2 + (1/n) sum of x_m over the m of j's parity
+//   Im a_j = -(H x)_j,  (H x)_j = (1/n) sum over odd d = j - m of cot(pi d / n) x_m
+// and for the FWI filter the complex conjugate of that, so
+//   Re(a b) = Re a Re b - Hx Hy (RTM), + Hx Hy (FWI).
+// H is a real Toeplitz operator that takes the odd cells to the even ones and back, so the column's
+// even cells and its odd cells are each one circular convolution of length L = the power of two >= nz,
+// and a field pair (x, y) goes through it as the complex column x + iy: 2 forward and 2 inverse
+// transforms of length L a field pair, where transforming each padded column by itself took 16 of
+// length >= 4nz - 1 (Bluestein's algorithm, which any nz that is not a power of two needed). x and y
+// may differ by orders of magnitude (a saved V^2/B-scaled derivative against a pressure), and a
+// transform rounds relative to the larger of the two it carries, so each is first brought to a maximum
+// of about 1 by a power of two of its own: without that the result was 1.7e-6 off at 40:1, with it
+// MEASURED_ERR.
+//
+// One thread holds 8 points of both transforms (u: odd cells, v: even cells), L/8 threads a column.
+// Stages are radix 8 (the last one 2 or 4 when log2 L is no multiple of 3), decimation in frequency
+// forward and in time back, in place in shared memory (one padded exchange between stages), so no
+// reordering is needed and the product with the transformed operator happens in registers. Each
+// persistent CTA forms the twiddles and the transformed operator itself, once, in shared memory: no
+// tables in global memory, so calls on any streams and of any nz share nothing.
+//
+// Bound by shared-memory traffic and FP32 issue (about 90 kflop a column at nz = 300), not by the
+// 24 B/cell that have to move. A whole call (3D Iso, 160 x 128 x 300 cells, nz no power of two): 153 us;
+// one CTA a column with radix-2 stages and sincospif twiddles took 5580 us.
 #include "wfd_kernels.h"
-#include "wfd_alloc.h"
 
 namespace WFD_NS {
 using namespace wfd;
 
 namespace {
 
+__device__ __forceinline__ float2 add(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 sub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+__device__ __forceinline__ float2 cmulc(float2 a, float2 b) {  // a * conj(b)
+    return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
+}
+// a * (S i)
+template <int S>
+__device__ __forceinline__ float2 muli(float2 a) {
+    return S > 0 ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+}
 
-// in-place radix-2 FFT of length m (power of two) in shared memory: a[k] = sum_j a[j] e^{sign 2 pi i jk/m}
-__device__ void fft_pow2(float2 *a, int m, int sign) {
-    const int lg = 31 - __clz(m);
-    for (int i = threadIdx.x; i < m; i += blockDim.x) {
-        const int j = (int)(__brev((unsigned)i) >> (32 - lg));
-        if (i < j) {
-            const float2 t = a[i];
-            a[i] = a[j];
-            a[j] = t;
+// X_k = sum_r a_r e^{S 2 pi i r k / N}, natural order in and out
+template <int S>
+__device__ __forceinline__ void dft4(float2 &a0, float2 &a1, float2 &a2, float2 &a3) {
+    const float2 s0 = add(a0, a2), d0 = sub(a0, a2), s1 = add(a1, a3), d1 = muli<S>(sub(a1, a3));
+    a0 = add(s0, s1);
+    a1 = add(d0, d1);
+    a2 = sub(s0, s1);
+    a3 = sub(d0, d1);
+}
+// HALF: a[4..7] are zero
+template <int S, bool HALF>
+__device__ __forceinline__ void dft8(float2 (&a)[8]) {
+    constexpr float h = 0.70710678118654752f;
+    float2 b[8];
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        b[r] = HALF ? a[r] : add(a[r], a[r + 4]);
+        b[r + 4] = HALF ? a[r] : sub(a[r], a[r + 4]);
+    }
+    b[5] = make_float2(h * (b[5].x - S * b[5].y), h * (b[5].y + S * b[5].x));
+    b[6] = muli<S>(b[6]);
+    b[7] = make_float2(h * (-b[7].x - S * b[7].y), h * (-b[7].y + S * b[7].x));
+    dft4<S>(b[0], b[1], b[2], b[3]);
+    dft4<S>(b[4], b[5], b[6], b[7]);
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        a[2 * r] = b[r];
+        a[2 * r + 1] = b[r + 4];
+    }
+}
+
+template <int K>
+struct Sep {
+    static constexpr int L = 1 << K;           // transform length
+    static constexpr int T = L / 8;            // threads of a column
+    static constexpr int NT = T > 256 ? T : 256;
+    static constexpr int CPB = NT / T;         // columns at a time
+    static constexpr int NS = K / 3;           // radix-8 stages
+    static constexpr int REM = 1 << (K % 3);   // radix of the last stage, 1: none
+    static constexpr int BUF = L + T;          // floats2 of one padded transform
+    static constexpr bool BIG = K == 13;       // no room for all tables: formed as they are used
+    // shared memory (float2): transforms, operator (v, u), twiddles, DC values
+    static constexpr int O_G = 2 * CPB * BUF;
+    static constexpr int O_W = O_G + (BIG ? 1 : 2) * L;
+    static constexpr int O_DC = O_W + (BIG ? 0 : L);
+    static constexpr int O_MAX = O_DC + 2 * CPB;  // a warp's largest |x| and |y|
+    static constexpr size_t SMEM = sizeof(float2) * (size_t)(O_MAX + NT / 32);
+    static_assert(SMEM <= 227 * 1024, "shared memory of a CTA");
+
+    // length of the sub-transforms of stage s, and where its twiddles start: w[(r-1) M/8 + q] for
+    // e^{-2 pi i q r / M}
+    static constexpr int M(int s) { return L >> (3 * s); }
+    static constexpr int woff(int s) { return s == 0 ? 0 : woff(s - 1) + 7 * (M(s - 1) / 8); }
+
+    static __device__ __forceinline__ int pad(int i) { return i + (i >> 3); }
+
+    template <int ST>
+    static __device__ __forceinline__ float2 twiddle(const float2 *w, int q, int r) {
+        if (!BIG) return w[woff(ST) + (r - 1) * (M(ST) / 8) + q];
+        float s, c;
+        sincospif(-2.0f * (float)(q * r) / (float)M(ST), &s, &c);
+        return make_float2(c, s);
+    }
+
+    // position of element r of this thread's butterfly in stage ST
+    template <int ST>
+    static __device__ __forceinline__ int pos(int t, int r) {
+        constexpr int P = M(ST) / 8;
+        return pad((t / P) * M(ST) + t % P + r * P);
+    }
+
+    template <bool V>
+    static __device__ __forceinline__ void rem(float2 (&a)[8]) {
+        constexpr int S = V ? 1 : -1;
+        if (REM == 4) {
+            dft4<S>(a[0], a[1], a[2], a[3]);
+            dft4<S>(a[4], a[5], a[6], a[7]);
+        } else if (REM == 2) {
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+                const float2 x = a[e], y = a[e + 1];
+                a[e] = add(x, y);
+                a[e + 1] = sub(x, y);
+            }
         }
     }
-    __syncthreads();
-    for (int half = 1; half < m; half <<= 1) {
-        const int len = half << 1;
-        for (int t = threadIdx.x; t < m / 2; t += blockDim.x) {
-            const int pos = t & (half - 1);
-            const int i = (t / half) * len + pos;
-            const int j = i + half;
-            float s, c;
-            sincospif((float)(2 * pos) / (float)len, &s, &c);
-            const float2 w = make_float2(c, sign * s);
-            const float2 u = a[i];
-            const float2 v = cmul(a[j], w);
-            a[i] = make_float2(u.x + v.x, u.y + v.y);
-            a[j] = make_float2(u.x - v.x, u.y - v.y);
+
+    // both transforms forward from stage ST (inputs in registers); afterwards register e holds
+    // position 8t + e
+    template <int ST, bool HALF>
+    static __device__ __forceinline__ void forward(float2 (&u)[8], float2 (&v)[8], float2 *bu, float2 *bv,
+                                                   const float2 *w, int t) {
+        if constexpr (ST < NS) {
+            dft8<-1, HALF>(u);
+            dft8<-1, HALF>(v);
+            constexpr int P = M(ST) / 8;
+            if constexpr (P > 1) {
+                const int q = t % P;
+#pragma unroll
+                for (int r = 1; r < 8; r++) {
+                    const float2 z = twiddle<ST>(w, q, r);
+                    u[r] = cmul(u[r], z);
+                    v[r] = cmul(v[r], z);
+                }
+                exchange<ST, ST + 1>(u, v, bu, bv, t);
+                forward<ST + 1, false>(u, v, bu, bv, w, t);
+            }
+        } else {
+            rem<false>(u);
+            rem<false>(v);
+        }
+    }
+
+    // back, from the registers forward() leaves to those it was given
+    template <int ST>
+    static __device__ __forceinline__ void inverse(float2 (&u)[8], float2 (&v)[8], float2 *bu, float2 *bv,
+                                                   const float2 *w, int t) {
+        if constexpr (ST == NS) {
+            rem<true>(u);
+            rem<true>(v);
+            if constexpr (REM > 1) exchange<NS, NS - 1>(u, v, bu, bv, t);
+            inverse<NS - 1>(u, v, bu, bv, w, t);
+        } else {
+            constexpr int P = M(ST) / 8;
+            if constexpr (P > 1) {
+                const int q = t % P;
+#pragma unroll
+                for (int r = 1; r < 8; r++) {
+                    const float2 z = twiddle<ST>(w, q, r);
+                    u[r] = cmulc(u[r], z);
+                    v[r] = cmulc(v[r], z);
+                }
+            }
+            dft8<1, false>(u);
+            dft8<1, false>(v);
+            if constexpr (ST > 0) {
+                exchange<ST, ST - 1>(u, v, bu, bv, t);
+                inverse<ST - 1>(u, v, bu, bv, w, t);
+            }
+        }
+    }
+
+    // stage FROM's outputs to the threads that need them in stage TO (in place; stage NS holds 8
+    // consecutive positions a thread)
+    template <int FROM, int TO>
+    static __device__ __forceinline__ void exchange(float2 (&u)[8], float2 (&v)[8], float2 *bu, float2 *bv, int t) {
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const int i = slot<FROM>(t, r);
+            bu[i] = u[r];
+            bv[i] = v[r];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const int i = slot<TO>(t, r);
+            u[r] = bu[i];
+            v[r] = bv[i];
+        }
+    }
+    template <int ST>
+    static __device__ __forceinline__ int slot(int t, int r) {
+        if constexpr (ST < NS) return pos<ST>(t, r);
+        else return pad(8 * t + r);
+    }
+
+    // frequency that forward() leaves at position p
+    static __device__ __forceinline__ int freq(int p) {
+        int f = 0, mul = 1;
+        for (int m = L; m > REM; m >>= 3) {
+            f += (p / (m / 8)) * mul;
+            p %= m / 8;
+            mul *= 8;
+        }
+        return f + p * mul;
+    }
+
+    // biased exponents of the column's largest |x| and |y| (1..253; 127 when it is not finite)
+    static __device__ __forceinline__ uint2 exponents(uint2 mx, uint2 *buf, int slot, int t) {
+        if constexpr (T >= 32) {
+            mx.x = __reduce_max_sync(0xffffffffu, mx.x);
+            mx.y = __reduce_max_sync(0xffffffffu, mx.y);
+            if constexpr (T > 32) {
+                if (t % 32 == 0) buf[(slot * T + t) / 32] = mx;
+                __syncthreads();
+                for (int i = 0; i < T / 32; i++) {
+                    const uint2 o = buf[slot * (T / 32) + i];
+                    mx.x = max(mx.x, o.x);
+                    mx.y = max(mx.y, o.y);
+                }
+            }
+        } else {
+            for (int o = T / 2; o > 0; o >>= 1) {
+                mx.x = max(mx.x, __shfl_xor_sync(0xffffffffu, mx.x, o));
+                mx.y = max(mx.y, __shfl_xor_sync(0xffffffffu, mx.y, o));
+            }
+        }
+        auto e = [](unsigned m) { return m >= 0x7f800000u ? 127u : min(max(m >> 23, 1u), 253u); };
+        return make_uint2(e(mx.x), e(mx.y));
+    }
+
+    // (1/L) cot(pi d / n) for the odd d that a column of nz cells reaches, else 0
+    static __device__ __forceinline__ float tap(int d, int nz) {
+        if (d >= nz || d <= -nz) return 0.0f;
+        double s, c;
+        sincospi((double)d / (2.0 * nz), &s, &c);
+        return (float)(c / s / L);
+    }
+};
+
+template <int K>
+__global__ void __launch_bounds__(Sep<K>::NT, Sep<K>::NT > 512 ? 1 : (Sep<K>::NT > 256 ? 1 : 3))
+    k_wavefieldsep(long ncols, int nz, int isfwi, const float *__restrict__ v_, const float *__restrict__ b_,
+                   const float *__restrict__ pold, const float *__restrict__ mold, const float *__restrict__ dp,
+                   const float *__restrict__ dm, float *__restrict__ dv) {
+    using C = Sep<K>;
+    constexpr int T = C::T, L = C::L;
+    extern __shared__ float2 sm[];
+    const int slot = threadIdx.x / T, t = threadIdx.x % T;
+    float2 *bu = sm + (2 * slot) * C::BUF, *bv = bu + C::BUF;
+    float2 *G = sm + C::O_G, *W = sm + C::O_W, *dc = sm + C::O_DC + 2 * slot;
+
+    // twiddles, then the operator's taps through the same transform
+    if (!C::BIG) {
+        for (int i = threadIdx.x; i < L; i += C::NT) {
+            int m = L, o = i;  // stage length and offset inside the stage
+            while (m >= 8 && o >= 7 * (m / 8)) {
+                o -= 7 * (m / 8);
+                m >>= 3;
+            }
+            if (m >= 8) {
+                const int r = o / (m / 8) + 1, q = o % (m / 8);
+                double s, c;
+                sincospi(-2.0 * (q * r) / m, &s, &c);
+                W[i] = make_float2((float)c, (float)s);
+            }
         }
         __syncthreads();
     }
-}
-
-struct SepTables {
-    const float2 *chirp;  // e^{+i pi j^2 / n}, j < n (Bluestein only)
-    const float2 *vplus;  // FFT_M of the conjugate chirp filter for sign +1
-    const float2 *vminus; // same for sign -1
-    int n, m;             // transform length and Bluestein length (m = 0: radix-2)
-};
-
-// buf[0..n) <- DFT_n(buf) with the given sign; bb is an m-long scratch for Bluestein
-__device__ void dft_n(float2 *buf, float2 *bb, const SepTables &T, int sign) {
-    if (T.m == 0) {
-        fft_pow2(buf, T.n, sign);
-        return;
-    }
-    const int n = T.n, m = T.m;
-    for (int j = threadIdx.x; j < m; j += blockDim.x) {
-        if (j < n) {
-            float2 c = T.chirp[j];
-            if (sign < 0) c.y = -c.y;
-            bb[j] = cmul(buf[j], c);
-        } else {
-            bb[j] = make_float2(0.0f, 0.0f);
+    {
+        float2 u[8], v[8];
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const int i = t + r * T, k = i < L / 2 ? i : i - L;
+            v[r] = make_float2(C::tap(2 * k + 1, nz), 0.0f);
+            u[r] = make_float2(C::tap(2 * k - 1, nz), 0.0f);
         }
-    }
-    __syncthreads();
-    fft_pow2(bb, m, -1);
-    const float2 *V = sign > 0 ? T.vplus : T.vminus;
-    for (int j = threadIdx.x; j < m; j += blockDim.x) bb[j] = cmul(bb[j], V[j]);
-    __syncthreads();
-    fft_pow2(bb, m, +1);
-    const float inv = 1.0f / (float)m;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        float2 c = T.chirp[k];
-        if (sign < 0) c.y = -c.y;
-        const float2 y = make_float2(bb[k].x * inv, bb[k].y * inv);
-        buf[k] = cmul(y, c);
-    }
-    __syncthreads();
-}
-
-__global__ void __launch_bounds__(256) k_wavefieldsep(Grid g, long isfwi, Fields F, const float *__restrict__ dp,
-                                                      const float *__restrict__ dm, float *dv, SepTables T, long col0) {
-    extern __shared__ float2 sm[];
-    const int n = T.n;
-    const int nz = (int)g.nz;
-    float2 *buf = sm;                          // n
-    float2 *res = buf + n;                     // nz
-    float *acc = (float *)(res + nz);          // nz
-    float2 *bb = (float2 *)(acc + nz + (nz & 1));  // m (Bluestein)
-    const long col = col0 + blockIdx.x;
-    if (col >= g.nx * g.ny) return;
-    const long base = col * g.nz;
-    const float scale = 1.0f / (float)n;
-    const int kadj = isfwi ? 0 : n / 2;
-    for (int z = threadIdx.x; z < nz; z += blockDim.x) acc[z] = 0.0f;
-    const int nfield = dm ? 2 : 1;
-    for (int fld = 0; fld < nfield; fld++) {
-        const float *nlf = fld == 0 ? dp : dm;
-        const float *adj = fld == 0 ? F.pold : F.mold;
-        for (int pass = 0; pass < 2; pass++) {
-            const float *src = pass == 0 ? nlf : adj;
-            for (int j = threadIdx.x; j < n; j += blockDim.x)
-                buf[j] = make_float2(j < nz ? scale * src[base + j] : 0.0f, 0.0f);
-            __syncthreads();
-            dft_n(buf, bb, T, +1);
-            const int z0 = pass == 0 ? n / 2 : kadj;  // up-going: drop positive bins; down-going: negative
-            for (int k = 1 + threadIdx.x; k < n / 2; k += blockDim.x) buf[z0 + k] = make_float2(0.0f, 0.0f);
-            __syncthreads();
-            dft_n(buf, bb, T, -1);
-            for (int z = threadIdx.x; z < nz; z += blockDim.x) {
-                if (pass == 0) res[z] = buf[z];
-                else acc[z] += res[z].x * buf[z].x - res[z].y * buf[z].y;
+        C::template forward<0, false>(u, v, bu, bv, W, t);
+        if (slot == 0) {
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                G[e * T + t] = v[e];
+                if (!C::BIG) G[L + e * T + t] = u[e];
             }
-            __syncthreads();
         }
+        __syncthreads();
     }
-    for (int z = threadIdx.x; z < nz; z += blockDim.x) {
-        const long k = base + z;
-        const float V = F.v[k];
-        const float B = F.b[k];
-        const float factor = 2 * B / (V * V * V);
-        dv[k] += factor * acc[z];
-    }
-}
 
-// host double-precision radix-2 FFT for the Bluestein filter tables
-void host_fft(std::vector<double> &re, std::vector<double> &im, int sign) {
-    const size_t m = re.size();
-    for (size_t i = 1, j = 0; i < m; i++) {
-        size_t bit = m >> 1;
-        for (; j & bit; bit >>= 1) j ^= bit;
-        j ^= bit;
-        if (i < j) {
-            std::swap(re[i], re[j]);
-            std::swap(im[i], im[j]);
+    const float scale = 1.0f / (float)(2 * nz);  // the reference rounds its scaled inputs: so here
+    const double sign = isfwi ? 1.0 : -1.0;
+    uint2 *red = reinterpret_cast<uint2 *>(sm + C::O_MAX);
+    const long ngroups = (ncols + C::CPB - 1) / C::CPB;
+    for (long cg = blockIdx.x; cg < ngroups; cg += gridDim.x) {
+        const long col = cg * C::CPB + slot;
+        const bool live = col < ncols;
+        const long base = col * nz;
+        // cells 2i and 2i + 1, i = t + r T; the sum and the image's increment in double, so that only
+        // the transforms' rounding is left in it
+        double acc[4][2];
+#pragma unroll
+        for (int r = 0; r < 4; r++) acc[r][0] = acc[r][1] = 0.0;
+        const int nfield = dm ? 2 : 1;
+        for (int fld = 0; fld < nfield; fld++) {
+            const float *x = (fld == 0 ? dp : dm) + base, *y = (fld == 0 ? pold : mold) + base;
+            float2 u[8], v[8];
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const int j = 2 * (t + r * T);
+                const bool in0 = live && j < nz, in1 = live && j + 1 < nz;
+                v[r] = make_float2(in0 ? scale * x[j] : 0.0f, in0 ? scale * y[j] : 0.0f);
+                u[r] = make_float2(in1 ? scale * x[j + 1] : 0.0f, in1 ? scale * y[j + 1] : 0.0f);
+                v[r + 4] = u[r + 4] = make_float2(0.0f, 0.0f);
+            }
+            uint2 mx = make_uint2(0u, 0u);
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                mx.x = max(mx.x, max(__float_as_uint(fabsf(u[r].x)), __float_as_uint(fabsf(v[r].x))));
+                mx.y = max(mx.y, max(__float_as_uint(fabsf(u[r].y)), __float_as_uint(fabsf(v[r].y))));
+            }
+            const uint2 ex = C::exponents(mx, red, slot, t);
+            const float2 norm = make_float2(__uint_as_float((254u - ex.x) << 23), __uint_as_float((254u - ex.y) << 23));
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                u[r] = make_float2(u[r].x * norm.x, u[r].y * norm.y);
+                v[r] = make_float2(v[r].x * norm.x, v[r].y * norm.y);
+            }
+            C::template forward<0, true>(u, v, bu, bv, W, t);
+            if (t == 0) {
+                dc[0] = v[0];
+                dc[1] = u[0];
+            }
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                const float2 gv = G[e * T + t];
+                float2 gu;
+                if (!C::BIG) {
+                    gu = G[L + e * T + t];
+                } else {  // the u taps are the v taps one place on
+                    float s, c;
+                    sincospif(-2.0f * (float)C::freq(8 * t + e) / (float)L, &s, &c);
+                    gu = cmul(gv, make_float2(c, s));
+                }
+                v[e] = cmul(v[e], gv);
+                u[e] = cmul(u[e], gu);
+            }
+            C::template inverse<(C::REM > 1 ? C::NS : C::NS - 1)>(u, v, bu, bv, W, t);
+            const float2 s0 = dc[0], s1 = dc[1];
+            // 2^e of the two normalisations, and Re a Re b -+ Hx Hy of one cell
+            const double ux = __hiloint2double((int)(ex.x + 896u) << 20, 0), uy = __hiloint2double((int)(ex.y + 896u) << 20, 0);
+            auto term = [&](float x, float y, float2 sum, float2 h) {
+                return ((double)nz * (scale * x) + ux * sum.x) * ((double)nz * (scale * y) + uy * sum.y) +
+                       sign * (ux * h.x) * (uy * h.y);
+            };
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const int j = 2 * (t + r * T);
+                if (live && j < nz)  // even cells: H of the odd ones (u)
+                    acc[r][0] += term(x[j], y[j], s0, u[r]);
+                if (live && j + 1 < nz) acc[r][1] += term(x[j + 1], y[j + 1], s1, v[r]);
+            }
         }
-    }
-    for (size_t len = 2; len <= m; len <<= 1) {
-        const double ang = sign * 2.0 * M_PI / (double)len;
-        for (size_t i = 0; i < m; i += len)
-            for (size_t k = 0; k < len / 2; k++) {
-                const double c = cos(ang * k), s = sin(ang * k);
-                const size_t a = i + k, b = i + k + len / 2;
-                const double vr = re[b] * c - im[b] * s, vi = re[b] * s + im[b] * c;
-                re[b] = re[a] - vr;
-                im[b] = im[a] - vi;
-                re[a] += vr;
-                im[a] += vi;
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int j = 2 * (t + r * T) + h;
+                if (live && j < nz) {
+                    const long k = base + j;
+                    const double V = v_[k];
+                    const double B = b_[k];
+                    dv[k] = (float)((double)dv[k] + 2 * B / (V * V * V) * acc[r][h]);
+                }
             }
     }
+}
+
+template <int K>
+bool launch(const Grid &g, long isfwi, const Fields &F, const float *dp, const float *dm, float *dv, cudaStream_t s) {
+    using C = Sep<K>;
+    const long ncols = g.nx * g.ny;
+    if (cudaFuncSetAttribute(k_wavefieldsep<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM) != cudaSuccess)
+        return false;
+    int dev = 0, sms = 0, per = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_wavefieldsep<K>, C::NT, C::SMEM) != cudaSuccess || per < 1)
+        return false;
+    const long groups = (ncols + C::CPB - 1) / C::CPB, cap = (long)sms * per;
+    k_wavefieldsep<K><<<(unsigned)(groups < cap ? groups : cap), C::NT, C::SMEM, s>>>(
+        ncols, (int)g.nz, isfwi ? 1 : 0, F.v, F.b, F.pold, F.mold, dp, dm, dv);
+    return true;
 }
 
 }  // namespace
 
-// Launch with Bluestein tables already on the device ({chirp[n], filter(+1)[m], filter(-1)[m]},
-// m = 0 for power-of-two n); allocates nothing.
-void image_wavefieldsep_tables(const Grid &g, long isfwi, const Fields &F, const float *dp, const float *dm,
-                               float *dv, const float2 *tables, int m, cudaStream_t s) {
-    const int n = (int)(2 * g.nz);
-    SepTables T{nullptr, nullptr, nullptr, n, m};
-    if (m) {
-        T.chirp = tables;
-        T.vplus = tables + n;
-        T.vminus = tables + n + m;
+bool image_wavefieldsep(const Grid &g, long isfwi, const Fields &F, const float *dp, const float *dm, float *dv,
+                        cudaStream_t s) {
+    int k = 4;
+    while (k < 14 && (1L << k) < g.nz + (g.nz & 1)) k++;
+    switch (k) {
+        case 4: return launch<4>(g, isfwi, F, dp, dm, dv, s);
+        case 5: return launch<5>(g, isfwi, F, dp, dm, dv, s);
+        case 6: return launch<6>(g, isfwi, F, dp, dm, dv, s);
+        case 7: return launch<7>(g, isfwi, F, dp, dm, dv, s);
+        case 8: return launch<8>(g, isfwi, F, dp, dm, dv, s);
+        case 9: return launch<9>(g, isfwi, F, dp, dm, dv, s);
+        case 10: return launch<10>(g, isfwi, F, dp, dm, dv, s);
+        case 11: return launch<11>(g, isfwi, F, dp, dm, dv, s);
+        case 12: return launch<12>(g, isfwi, F, dp, dm, dv, s);
+        case 13: return launch<13>(g, isfwi, F, dp, dm, dv, s);
+        default: return false;  // deeper than 8192 cells: no CTA's shared memory holds a column
     }
-    const long nz = g.nz;
-    const size_t smem = sizeof(float2) * (size_t)n + sizeof(float2) * (size_t)nz +
-                        sizeof(float) * (size_t)(nz + (nz & 1)) + sizeof(float2) * (size_t)m;
-    cudaFuncSetAttribute(k_wavefieldsep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const long ncols = g.nx * g.ny;
-    const long chunk = 65535;
-    for (long c0 = 0; c0 < ncols; c0 += chunk) {
-        const long nb = ncols - c0 < chunk ? ncols - c0 : chunk;
-        k_wavefieldsep<<<(unsigned)nb, 256, smem, s>>>(g, isfwi, F, dp, dm, dv, T, c0);
-    }
-}
-
-void image_wavefieldsep(const Grid &g, long isfwi, const Fields &F, const float *dp, const float *dm, float *dv,
-                        float2 *work, long ncols_per_pass, cudaStream_t s) {
-    (void)work;
-    (void)ncols_per_pass;
-    const int n = (int)(2 * g.nz);
-    const bool pow2 = (n & (n - 1)) == 0;
-    int m = 0;
-    SepTables T{nullptr, nullptr, nullptr, n, 0};
-    float2 *tables = nullptr;
-    if (!pow2) {
-        m = 1;
-        while (m < 2 * n - 1) m <<= 1;
-        T.m = m;
-        std::vector<float2> h((size_t)n + 2 * (size_t)m);
-        std::vector<double> cr(n), ci(n);
-        for (long j = 0; j < n; j++) {
-            const long q = (j * j) % (2L * n);  // exact phase pi*j^2/n reduced mod 2 pi
-            cr[j] = cos(M_PI * (double)q / (double)n);
-            ci[j] = sin(M_PI * (double)q / (double)n);
-            h[j] = make_float2((float)cr[j], (float)ci[j]);
-        }
-        for (int sgn = 0; sgn < 2; sgn++) {
-            const double sg = sgn == 0 ? 1.0 : -1.0;
-            std::vector<double> vr(m, 0.0), vi(m, 0.0);
-            for (long j = 0; j < n; j++) {
-                // conj(c_s[j]) with c_s = e^{s i pi j^2/n}
-                vr[j] = cr[j];
-                vi[j] = -sg * ci[j];
-                if (j > 0) {
-                    vr[m - j] = vr[j];
-                    vi[m - j] = vi[j];
-                }
-            }
-            host_fft(vr, vi, -1);
-            for (int j = 0; j < m; j++) h[(size_t)n + (size_t)sgn * m + j] = make_float2((float)vr[j], (float)vi[j]);
-        }
-        wfd::dMallocAsync(&tables, sizeof(float2) * h.size(), s);
-        cudaMemcpyAsync(tables, h.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice, s);
-        T.chirp = tables;
-        T.vplus = tables + n;
-        T.vminus = tables + n + m;
-    }
-    const long nz = g.nz;
-    size_t smem = sizeof(float2) * (size_t)n + sizeof(float2) * (size_t)nz + sizeof(float) * (size_t)(nz + (nz & 1));
-    smem += sizeof(float2) * (size_t)m;
-    cudaFuncSetAttribute(k_wavefieldsep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const long ncols = g.nx * g.ny;
-    const long chunk = 65535;
-    for (long c0 = 0; c0 < ncols; c0 += chunk) {
-        const long nb = ncols - c0 < chunk ? ncols - c0 : chunk;
-        k_wavefieldsep<<<(unsigned)nb, 256, smem, s>>>(g, isfwi, F, dp, dm, dv, T, c0);
-    }
-    if (tables) cudaFreeAsync(tables, s);
 }
 
 }  // namespace WFD_NS
