@@ -95,14 +95,14 @@ extern "C" int WFD_Prop_Prefetch(void *p) {
     if (!p) return WFD_ERR_ARG;
     Prop *q = P(p);
     q->host_touched = 0;
-    const size_t bytes = sizeof(float) * (size_t)q->ncells();
+    const size_t bytes = q->alloc_bytes();
     for (int f = 0; f < wfd::F_COUNT; f++) {
-        if (!q->field[f]) continue;
+        if (!q->alloc[f]) continue;
 #if CUDART_VERSION >= 13000
         cudaMemLocation loc{cudaMemLocationTypeDevice, q->device};
-        cudaMemPrefetchAsync(q->field[f], bytes, loc, 0, q->stream);
+        cudaMemPrefetchAsync(q->alloc[f], bytes, loc, 0, q->stream);
 #else
-        cudaMemPrefetchAsync(q->field[f], bytes, q->device, q->stream);
+        cudaMemPrefetchAsync(q->alloc[f], bytes, q->device, q->stream);
 #endif
     }
     return wfd::prop_sync(q);

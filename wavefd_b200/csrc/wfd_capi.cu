@@ -37,7 +37,7 @@ namespace wfd {
 void prefetch_touched(Prop *p, cudaStream_t s) {
     const unsigned mask = p->host_touched;
     p->host_touched = 0;
-    const size_t bytes = sizeof(float) * (size_t)p->ncells();
+    const size_t bytes = p->alloc_bytes(), margin = field_margin(p->ndim, p->phys, p->nz);
     for (int f = 0; f < F_COUNT; f++) {
         if (!(mask >> f & 1u)) {
             p->touch_streak[f] = 0;
@@ -48,9 +48,9 @@ void prefetch_touched(Prop *p, cudaStream_t s) {
         if (again || !p->field[f]) continue;
 #if CUDART_VERSION >= 13000
         cudaMemLocation loc{cudaMemLocationTypeDevice, p->device};
-        cudaMemPrefetchAsync(p->field[f], bytes, loc, 0, s);
+        cudaMemPrefetchAsync(p->field[f] - margin, bytes, loc, 0, s);
 #else
-        cudaMemPrefetchAsync(p->field[f], bytes, p->device, s);
+        cudaMemPrefetchAsync(p->field[f] - margin, bytes, p->device, s);
 #endif
     }
 }

@@ -6,7 +6,7 @@ using namespace wfd;
 
 int fused_step(const Grid &g, int phys, int linear, const Fields &F, cudaStream_t s) {
     Fields Fn = F;
-    Fn.illum = nullptr;      // the TMA-staged Iso, VTI and TTI kernels accumulate the illumination
+    Fn.illum = nullptr;      // the TMA-staged 3D kernels accumulate the illumination
     Fn.inj.ngroups = 0;      // themselves; only the 2D Iso kernel applies a source injection itself
     Fn.epi = StepEpilogue{};  // and only the TMA-staged 3D kernels apply the Born/imaging epilogue
     Fields Fl = Fn;
@@ -16,10 +16,9 @@ int fused_step(const Grid &g, int phys, int linear, const Fields &F, cudaStream_
     const int lit = F.illum ? 2 : 0;
     const int ept = (F.epi.born_dv || F.epi.img || F.epi.scale_space) ? 8 : 0;
     if (g.ndim == 3 && phys == ISO) {
-        // TMA-staged kernel when the tensor maps can be encoded (nz*4 a multiple of 16 bytes),
-        // else the variant that stages its tiles with ordinary loads
-        if (fused_iso3d_tma(g, Fe, s)) return 1 | lit | ept;
-        return fused_iso3d(g, Fn, s) ? 1 : 0;
+        // one kernel, tiles staged by TMA (nz*4 a multiple of 16 bytes) or by cp.async
+        const int r = fused_iso3d_tma(g, Fe, s);
+        return r == 2 ? 1 | lit | ept : r;
     }
     if (g.ndim == 3 && phys == VTI) {
         // the VTI kernel with x-direction register queues, else the ring-staged kernel TTI uses

@@ -22,6 +22,7 @@
 // to it as the cell is updated. Waits are bounded; on timeout the kernel records an error in a device status
 // word and leaves. Requires nz % 4 == 0 (TMA row pitch); the caller falls back otherwise.
 #include "wfd_kernels.h"
+#include "wfd_ragged.cuh"
 #include "wfd_tma.cuh"
 
 namespace WFD_NS {
@@ -220,10 +221,10 @@ __device__ __forceinline__ void ext_stage(const Grid &g, const bool xin, const b
 
 // D- in y and z, the time update and the stores of this thread's 4 cells (fmask bit m: the
 // reference updates cell m, given x)
-template <int MODE, bool EPI>
+template <int MODE, bool EPI, bool RAG>
 __device__ __forceinline__ void fin_stage(const Grid &g, const long j, const bool xin, const bool top, const int z,
                                           const int y, const unsigned fmask, const int zq, const int row,
-                                          const float2 *sx, const float2 *pc, const float *st, const float *TYs,
+                                          const float2 *sx, const float2 *pc, float *st, const float *TYs,
                                           const float *TZs, float *po, float *ps, float *illum,
                                           const StepEpilogue *epi, const float4 ea, const float4 eb) {
     const int o = row * TZ + 4 * zq;
@@ -301,6 +302,13 @@ __device__ __forceinline__ void fin_stage(const Grid &g, const long j, const boo
         npo[h] = np;
         nps[h] = nl;
     }
+    if (RAG) {
+        // rows start at any alignment: the results go through this thread's own pOld and V cells of
+        // the stage, and the warp stores its rows 32 columns at a time (ragged_store)
+        st4(st + S_PO + o, make_float4(npo[0].x, npo[0].y, npo[1].x, npo[1].y));
+        st4(st + S_V + o, make_float4(nps[0].x, nps[0].y, nps[1].x, nps[1].y));
+        return;
+    }
     const long k = j * g.sx + (long)y * g.nz + z;
     st4(po + k, make_float4(npo[0].x, npo[0].y, npo[1].x, npo[1].y));
     st4(ps + k, make_float4(nps[0].x, nps[0].y, nps[1].x, nps[1].y));
@@ -313,6 +321,21 @@ __device__ __forceinline__ void fin_stage(const Grid &g, const long j, const boo
         a.z = __fadd_rn(a.z, __fmul_rn(pc[1].x, pc[1].x));
         a.w = __fadd_rn(a.w, __fmul_rn(pc[1].y, pc[1].y));
         st4(illum + k, a);
+    }
+}
+
+// the warp's 4 rows of new pOld and pSpace values from the stage to the arrays, a row at a time
+__device__ __forceinline__ void ragged_store(const Grid &g, const long j, const int z0, const int y0, const float *st,
+                                             float *po, float *ps) {
+    const int lane = threadIdx.x & 31, r0 = 4 * (threadIdx.x >> 5);
+    __syncwarp();
+    const long k = j * g.sx + (long)(y0 + r0) * g.nz + z0 + lane;
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        if (z0 + lane < g.nz && y0 + r0 + r < g.ny) {
+            po[k + r * g.nz] = st[S_PO + (r0 + r) * TZ + lane];
+            ps[k + r * g.nz] = st[S_V + (r0 + r) * TZ + lane];
+        }
     }
 }
 
@@ -347,7 +370,11 @@ __device__ __forceinline__ void queue_phase(float2 (&qp)[8][2], float2 (&qt)[8][
 // BATCH = true: many objects (shots) of different sizes; every item names its shot, whose sizes,
 // output pointers and tensor maps sit in a descriptor in global memory; CTAs take items from a
 // shared counter (dynamic scheduling over shots of uneven size, in the order the caller packed).
-template <bool BATCH, bool EPI = false>
+// RAG = true: rows that TMA cannot address (nz % 4 != 0), staged by every thread's cp.async
+// (wfd_ragged.cuh) into the same boxes; single objects, no epilogue and no illumination. 301 x 203 x 251:
+// 180 us a step, 617 us by the kernel that it took the place of (tiles staged through registers with one
+// plane of 256 threads and no overlap).
+template <bool BATCH, bool EPI = false, bool RAG = false>
 __global__ void __launch_bounds__(NT, 3)
     k_iso3d_tma(Grid g0, Fields F, const __grid_constant__ IsoMaps M, int ntz0, int nty0, int nch0, int xchunk0,
                 const IsoShotDesc *__restrict__ shots, const int *__restrict__ sel, const int2 *__restrict__ items,
@@ -363,9 +390,9 @@ __global__ void __launch_bounds__(NT, 3)
     const int lane = tid & 31;
     const int warp = tid >> 5;
     if (tid == 0) {
-        for (int s = 0; s < NS; s++) mbar_init(&bars[s], 1);
+        for (int s = 0; s < NS; s++) mbar_init(&bars[s], RAG ? NT : 1);
         fence_mbar_init();
-        if (!BATCH)
+        if (!BATCH && !RAG)
             for (int i = 0; i < 7; i++) prefetch_tensor_map(&M.m[i]);
         *abort_flag = 0;
     }
@@ -431,9 +458,28 @@ __global__ void __launch_bounds__(NT, 3)
         }
         const unsigned emask = ext_mask(g, tid, z0, y0);
 
+        using BoxP = RaggedBox<PZW, PYH, NT / 32>;
+        using BoxB = RaggedBox<BZW, BYH, NT / 32>;
+        using BoxT = RaggedBox<TZ, TY, NT / 32>;
         auto issue = [&](long jj, unsigned gs) {
             uint64_t *bar = &bars[gs % NS];
             float *s = sm + (gs % NS) * STAGE;
+            if (RAG) {
+                const int nz = (int)g.nz;
+                auto plane = [&](const float *f, long x) { return f + min(max(x, 0l), g.nx - 1) * g.sx; };
+                BoxT::load(s + S_PN, plane(F.pcur, jj + 7), z0, y0, nz, warp, lane);
+                BoxT::load(s + S_BN, plane(F.b, jj + 3), z0, y0, nz, warp, lane);
+                if (jj >= xbeg) {  // the warm-up planes only fill the queues
+                    const long k = jj * g.sx;
+                    BoxP::load(s + S_PH, F.pcur + k, z0 - 8, y0 - 7, nz, warp, lane);
+                    BoxB::load(s + S_BH, F.b + k, z0 - 4, y0 - 4, nz, warp, lane);
+                    BoxT::load(s + S_PO, out_pold + k, z0, y0, nz, warp, lane);
+                    BoxT::load(s + S_V, F.v + k, z0, y0, nz, warp, lane);
+                    BoxT::load(s + S_Q, F.q + k, z0, y0, nz, warp, lane);
+                }
+                cp_async_arrive(bar);
+                return;
+            }
             mbar_expect_tx(bar, GROUP_BYTES);
             tma_load_3d(s + S_PH, mPH, bar, z0 - 8, y0 - 7, (int)jj);
             tma_load_3d(s + S_BH, mBH, bar, z0 - 4, y0 - 4, (int)jj);
@@ -443,7 +489,7 @@ __global__ void __launch_bounds__(NT, 3)
             tma_load_3d(s + S_V, mV, bar, z0, y0, (int)jj);
             tma_load_3d(s + S_Q, mQ, bar, z0, y0, (int)jj);
         };
-        if (tid == 0) {
+        if (RAG || tid == 0) {
             for (int q = 0; q < D && q < ngroups; q++) issue(jstart + q, gseq + q);
             out_from = gseq;
             out_to = gseq + (D < ngroups ? D : ngroups);
@@ -463,7 +509,7 @@ __global__ void __launch_bounds__(NT, 3)
         for (int q = 0; q < ngroups; q++) {
             const long j = jstart + q;
             const unsigned gs = gseq + q;
-            if (tid == 0 && q + D < ngroups) {
+            if ((RAG || tid == 0) && q + D < ngroups) {
                 issue(j + D, gs + D);
                 out_to = gs + D + 1;
             }
@@ -487,7 +533,7 @@ __global__ void __launch_bounds__(NT, 3)
             }
             // a group whose wait ran out may still be in flight: the drain below waits for it
             if (tid == 0 && landed) out_from = gs + 1;
-            const float *st = sm + slot * STAGE;
+            float *st = sm + slot * STAGE;
             slot = slot + 1 == NS ? 0u : slot + 1;
             par ^= slot == 0 ? 1u : 0u;
             float2 sx[2], pc[2];
@@ -512,8 +558,9 @@ __global__ void __launch_bounds__(NT, 3)
                 // one code path for every tile (the selects are cheap, code size is not)
                 ext_stage<EDGE>(g, xin, tile_top, z0, emask, st, TYs, TZs);
                 __syncthreads();
-                if (own) fin_stage<EDGE, EPI>(g, j, xin, tile_top, z, y, fmask, zq, row, sx, pc, st, TYs, TZs, out_pold,
+                if (own) fin_stage<EDGE, EPI, RAG>(g, j, xin, tile_top, z, y, fmask, zq, row, sx, pc, st, TYs, TZs, out_pold,
                                                out_pspace, BATCH ? nullptr : F.illum, EPI ? &F.epi : nullptr, ea, eb);
+                if (RAG) ragged_store(g, j, z0, y0, st, out_pold, out_pspace);
             }
             __syncthreads();
             if (*abort_flag) {
@@ -524,7 +571,9 @@ __global__ void __launch_bounds__(NT, 3)
         gseq += ngroups;
         if (stop) break;
     }
-    if (*abort_flag && tid == 0) {
+    if (RAG) {
+        cp_async_drain();
+    } else if (*abort_flag && tid == 0) {
         // let copies still in flight land before the CTA leaves (bounded)
         for (unsigned gs = out_from; gs < out_to; gs++) mbar_wait(&bars[gs % NS], (gs / NS) & 1u, 100000000ull);
     }
@@ -538,7 +587,7 @@ int iso_grid_cap() {
     static int cap = 0;
     if (!cap) {
         int dev = 0, sms = 0, per = 0;
-        for (auto kern : {k_iso3d_tma<false>, k_iso3d_tma<true>, k_iso3d_tma<false, true>})
+        for (auto kern : {k_iso3d_tma<false>, k_iso3d_tma<true>, k_iso3d_tma<false, true>, k_iso3d_tma<false, false, true>})
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -560,10 +609,10 @@ bool iso_maps(const Grid &g, const Fields &F, CUtensorMap *m) {
 
 }  // namespace
 
-bool fused_iso3d_tma(const Grid &g, const Fields &F, cudaStream_t s) {
-    if (g.nz % 4 != 0) return false;
+int fused_iso3d_tma(const Grid &g, const Fields &F, cudaStream_t s) {
     IsoMaps M;
-    if (!iso_maps(g, F, M.m)) return false;
+    const bool rag = g.nz % 4 != 0;  // (the arrays then have the margin that the ragged boxes need)
+    if (!rag && !iso_maps(g, F, M.m)) return 0;
     const int grid_cap = iso_grid_cap();
     const int ntz = (int)((g.nz + TZ - 1) / TZ);
     const int nty = (int)((g.ny + TY - 1) / TY);
@@ -585,13 +634,10 @@ bool fused_iso3d_tma(const Grid &g, const Fields &F, cudaStream_t s) {
     const int nch = (int)((g.nx + xchunk - 1) / xchunk);
     const long work = tiles * nch;
     const int grid = (int)(work < grid_cap ? work : grid_cap);
-if (F.epi.born_dv || F.epi.img || F.epi.scale_space)
-            k_iso3d_tma<false, true><<<grid, NT, SMEM_BYTES, s>>>(g, F, M, ntz, nty, nch, xchunk, nullptr, nullptr, nullptr, 0,
-                                                    nullptr);
-    else
-            k_iso3d_tma<false><<<grid, NT, SMEM_BYTES, s>>>(g, F, M, ntz, nty, nch, xchunk, nullptr, nullptr, nullptr, 0,
-                                                    nullptr);
-    return true;
+    const bool epi = F.epi.born_dv || F.epi.img || F.epi.scale_space;
+    auto *kern = rag ? k_iso3d_tma<false, false, true> : (epi ? k_iso3d_tma<false, true> : k_iso3d_tma<false>);
+    kern<<<grid, NT, SMEM_BYTES, s>>>(g, F, M, ntz, nty, nch, xchunk, nullptr, nullptr, nullptr, 0, nullptr);
+    return rag ? 1 : 2;
 }
 
 bool iso3d_tma_describe(const Grid &g, const Fields &F, int xchunk, IsoShotDesc *d, TileInfo *t) {

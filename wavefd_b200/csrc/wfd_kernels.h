@@ -107,7 +107,6 @@ struct TileInfo {
     void scale(const wfd::Grid &g, const wfd::Fields &F, bool two, cudaStream_t s);                      \
     void dplus3(const wfd::Grid &g, const float *inx, const float *iny, const float *inz, float *ox,     \
                 float *oy, float *oz, cudaStream_t s);                                                   \
-    bool fused_iso3d(const wfd::Grid &g, const wfd::Fields &F, cudaStream_t s);                          \
     bool fused_iso2d(const wfd::Grid &g, const wfd::Fields &F, cudaStream_t s);                          \
     bool fused_aniso2d(const wfd::Grid &g, int phys, int linear, const wfd::Fields &F, cudaStream_t s);  \
     /* whole 2D Iso time loop in one cooperative launch: 0 launched, -1 not available, 1 launch error */ \
@@ -116,7 +115,20 @@ struct TileInfo {
     /* the same for 2D VTI and TTI (phys), the tiles shared out over the co-resident CTAs */           \
     int aniso2d_run(const wfd::Grid &g, int phys, const wfd::Fields &F, long nsteps, long it0,          \
                     const wfd::RunExtract &ex, unsigned *sync_words, cudaStream_t s);                    \
-    bool fused_iso3d_tma(const wfd::Grid &g, const wfd::Fields &F, cudaStream_t s);                      \
+    bool fused_iso2d(const wfd::Grid &g, const wfd::Fields &F, cudaStream_t s);                          \
+    bool fused_aniso2d(const wfd::Grid &g, int phys, int linear, const wfd::Fields &F, cudaStream_t s);  \
+    /* whole 2D Iso time loop in one cooperative launch: 0 launched, -1 not available, 1 launch error */ \
+    int iso2d_run(const wfd::Grid &g, const wfd::Fields &F, long nsteps, long it0, const wfd::RunExtract &ex, \
+                  unsigned *sync_words, cudaStream_t s);                                                 \
+    /* the same for 2D VTI and TTI (phys), the tiles shared out over the co-resident CTAs */           \
+    int aniso2d_run(const wfd::Grid &g, int phys, const wfd::Fields &F, long nsteps, long it0,          \
+                    const wfd::RunExtract &ex, unsigned *sync_words, cudaStream_t s);                    \
+    /* 3D Iso: 0 not handled, 1 stepped (rows staged by cp.async: F.illum and F.epi not applied), 2    \
+       stepped with F.illum and F.epi */                                                                 \
+    int fused_iso3d_tma(const wfd::Grid &g, const wfd::Fields &F, cudaStream_t s);                       \
+    /* 3D Iso: 0 not handled, 1 stepped (ragged rows: F.illum and F.epi not applied), 2 stepped with     \
+       F.illum and F.epi */                                                                              \
+    int fused_iso3d_tma(const wfd::Grid &g, const wfd::Fields &F, cudaStream_t s);                       \
     bool fused_aniso3d_tma(const wfd::Grid &g, int phys, int linear, const wfd::Fields &F, cudaStream_t s); \
     bool fused_vti3d_tma(const wfd::Grid &g, int linear, const wfd::Fields &F, cudaStream_t s);         \
     bool vti3d_tma_describe(const wfd::Grid &g, const wfd::Fields &F, int xchunk, wfd::AnisoShotDesc *d, \

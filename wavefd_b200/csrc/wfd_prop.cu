@@ -82,6 +82,8 @@ static int check_cuda(Prop *p, cudaError_t e, const char *what) {
     return prop_fail(p, WFD_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+size_t Prop::alloc_bytes() const { return sizeof(float) * ((size_t)ncells() + 2 * field_margin(ndim, phys, nz)); }
+
 Grid Prop::grid() const {
     Grid g;
     g.ndim = ndim;
@@ -179,13 +181,16 @@ Prop *prop_create(int ndim, int phys, long fs, long nthread, long nx, long ny, l
     p->fused = !(fz && fz[0] == '1');
     cudaGetDevice(&p->device);
     // the arrays first, then the stream (an allocation failure is reported before any other call)
-    const size_t bytes = sizeof(float) * (size_t)p->ncells();
+    const size_t margin = field_margin(ndim, phys, nz);
+    const size_t bytes = p->alloc_bytes();
     for (int f = 0; f < F_COUNT; f++) {
         if (!uses(phys, ndim, f)) continue;
-        cudaError_t e = wfd::dMallocManaged(&p->field[f], bytes, cudaMemAttachGlobal);
+        cudaError_t e = wfd::dMallocManaged(&p->alloc[f], bytes, cudaMemAttachGlobal);
+        p->field[f] = p->alloc[f] + margin;
         if (e != cudaSuccess) {
             set_global_error(WFD_ERR_ALLOC, std::string("managed allocation failed: ") + cudaGetErrorString(e) +
                                                 alloc_injected_note());
+            p->alloc[f] = nullptr;
             prop_destroy(p);
             return nullptr;
         }
@@ -197,15 +202,15 @@ Prop *prop_create(int ndim, int phys, long fs, long nthread, long nx, long ny, l
     }
     p->own_stream = true;
     for (int f = 0; f < F_COUNT; f++) {
-        if (!p->field[f]) continue;
+        if (!p->alloc[f]) continue;
 #if CUDART_VERSION >= 13000
         cudaMemLocation loc{cudaMemLocationTypeDevice, p->device};
-        cudaMemAdvise(p->field[f], bytes, cudaMemAdviseSetPreferredLocation, loc);
+        cudaMemAdvise(p->alloc[f], bytes, cudaMemAdviseSetPreferredLocation, loc);
 #else
-        cudaMemAdvise(p->field[f], bytes, cudaMemAdviseSetPreferredLocation, p->device);
+        cudaMemAdvise(p->alloc[f], bytes, cudaMemAdviseSetPreferredLocation, p->device);
 #endif
         // the reference zero-fills every array at construction (numaFirstTouch, .h:94-205)
-        cudaMemsetAsync(p->field[f], 0, bytes, p->stream);
+        cudaMemsetAsync(p->alloc[f], 0, bytes, p->stream);
     }
     if (cudaStreamSynchronize(p->stream) != cudaSuccess) {
         set_global_error(WFD_ERR_CUDA, "initialisation failed");
@@ -219,7 +224,7 @@ void prop_destroy(Prop *p) {
     if (!p) return;
     if (p->stream) cudaStreamSynchronize(p->stream);
     for (int f = 0; f < F_COUNT; f++)
-        if (p->field[f]) cudaFree(p->field[f]);
+        if (p->alloc[f]) cudaFree(p->alloc[f]);
     for (int i = 0; i < 12; i++)
         if (p->tmp[i]) cudaFree(p->tmp[i]);
     for (int i = 0; i < 7; i++)

@@ -31,6 +31,7 @@ struct Prop {
     bool strict = false;     // bitwise parity kernels instead of the FMA build
     bool fused = true;       // single-sweep kernels where available
     float *field[F_COUNT] = {};
+    float *alloc[F_COUNT] = {};  // the allocations behind the fields (field = alloc + margin)
     float *tmp[12] = {};     // scratch of the unfused passes (the reference's tmp arrays)
     float *stage[7] = {};    // device copies of host arrays given to Born/imaging calls (first use)
     float *illum = nullptr;  // caller's source illumination sum (device), accumulated by every step
@@ -46,10 +47,18 @@ struct Prop {
     bool inject_done = false;  // the last step kernel applied `inj`
 
     long ncells() const { return nx * ny * nz; }
+    size_t alloc_bytes() const;  // of one field's allocation
     Grid grid() const;
     Fields fields() const;
     Scratch scratch() const;
 };
+
+// Floats before and after every field array of an object. The step kernel that stages ragged rows
+// (3D Iso, nz % 4 != 0) reads tile boxes without bounds tests: up to 7 rows and 8 columns before a plane and
+// 22 rows and 40 columns after one.
+inline size_t field_margin(int ndim, int phys, long nz) {
+    return ndim == 3 && phys == ISO && nz % 4 != 0 ? ((size_t)(32 * nz + 64) + 63) / 64 * 64 : 0;
+}
 
 Prop *prop_create(int ndim, int phys, long fs, long nthread, long nx, long ny, long nz, long nsponge, float dx,
                   float dy, float dz, float dt, long nbx, long nby, long nbz);
