@@ -10,7 +10,8 @@ from tests.harness import ABIRunner, OracleRunner, make_model, rel_l2, same
 pytestmark = pytest.mark.gpu
 
 NAMES = ["Prop3DAcoIsoDenQ_DEO2_FDTD", "Prop3DAcoVTIDenQ_DEO2_FDTD", "Prop3DAcoTTIDenQ_DEO2_FDTD"]
-SHAPES = [(9, 9, 9), (31, 15, 20), (33, 17, 40), (34, 16, 12), (35, 33, 17), (66, 18, 133)]  # (nz, ny, nx)
+SHAPES = [(9, 9, 9), (31, 15, 20), (33, 17, 40), (34, 16, 12), (35, 33, 17), (66, 18, 133),
+          (101, 98, 107), (103, 33, 301)]  # (nz, ny, nx); the last two take the marching two-pass kernels in VTI and TTI
 
 
 @pytest.fixture(scope="module")

@@ -31,7 +31,7 @@ STRICT = ["-DWFD_STRICT=1", "-fmad=false", "-prec-div=true", "-prec-sqrt=true", 
 FAST = ["-DWFD_STRICT=0", "-fmad=true", "-prec-div=false", "-prec-sqrt=false", "-ftz=true"]
 HOST = ["-Xcompiler", "-fopenmp"]  # host loops of the drop-in calls use the caller's thread count
 
-KERNEL_SOURCES = ["wfd_generic.cu", "wfd_fused.cu", "wfd_fused_iso3d_tma.cu",
+KERNEL_SOURCES = ["wfd_generic.cu", "wfd_pass3d.cu", "wfd_fused.cu", "wfd_fused_iso3d_tma.cu",
                   "wfd_fused_aniso3d_tma.cu", "wfd_fused_vti3d_tma.cu", "wfd_fused_iso2d.cu", "wfd_fused_aniso2d.cu",
                   "wfd_wavefieldsep.cu"]
 HOST_SOURCES = ["wfd_prop.cu", "wfd_bornimage.cu", "wfd_capi.cu", "wfd_addon.cu", "wfd_spacetime.cu",

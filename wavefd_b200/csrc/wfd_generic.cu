@@ -1,8 +1,8 @@
 // Unfused kernels: the reference's pass structure on the GPU, one thread per cell.
 //
 // These serve the Born-injection and imaging-condition entry points (which the reference
-// builds from standalone D+/D- passes and pointwise loops) and act as the unfused time step
-// for geometries the fused kernels do not take. Per-cell arithmetic follows the reference's
+// builds from standalone D+/D- passes and pointwise loops) and act as the unfused time step of 2D
+// and of small 3D grids (the larger ones: wfd_pass3d.cu) for geometries the fused kernels do not take. Per-cell arithmetic follows the reference's
 // expression trees; see the file:line notes at each kernel.
 #include "wfd_kernels.h"
 
@@ -570,6 +570,7 @@ MPtr3 m3(float *const *a) { return MPtr3{{a[0], a[1], a[2]}}; }
 
 // ---------------------------------------------------------------------------------------------
 void pass1(const Grid &g, int phys, const Fields &F, const Scratch &S, cudaStream_t s) {
+    if (pass3d_takes(g)) return pass1_3d(g, phys, F, S, s);
     const unsigned nb = blocks_for(g.n);
     if (phys == ISO) k_pass1<ISO><<<nb, kThreads, 0, s>>>(g, F, S);
     else if (phys == VTI) k_pass1<VTI><<<nb, kThreads, 0, s>>>(g, F, S);
@@ -577,6 +578,7 @@ void pass1(const Grid &g, int phys, const Fields &F, const Scratch &S, cudaStrea
 }
 
 void pass2(const Grid &g, int phys, int linear, const Fields &F, const Scratch &S, cudaStream_t s) {
+    if (pass3d_takes(g)) return pass2_3d(g, phys, linear, F, S, s);
     const unsigned nb = blocks_for(g.n);
     if (phys == ISO) k_pass2<ISO, false><<<nb, kThreads, 0, s>>>(g, F, S);
     else if (phys == VTI && linear) k_pass2<VTI, true><<<nb, kThreads, 0, s>>>(g, F, S);

@@ -100,6 +100,11 @@ struct TileInfo {
     void pass1(const wfd::Grid &g, int phys, const wfd::Fields &F, const wfd::Scratch &S, cudaStream_t s); \
     void pass2(const wfd::Grid &g, int phys, int linear, const wfd::Fields &F, const wfd::Scratch &S,    \
                cudaStream_t s);                                                                          \
+    /* the same two passes for the larger 3D grids (pass3d_takes) */                                     \
+    bool pass3d_takes(const wfd::Grid &g);                                                               \
+    void pass1_3d(const wfd::Grid &g, int phys, const wfd::Fields &F, const wfd::Scratch &S, cudaStream_t s); \
+    void pass2_3d(const wfd::Grid &g, int phys, int linear, const wfd::Fields &F, const wfd::Scratch &S, \
+                  cudaStream_t s);                                                                       \
     /* fused single-sweep steps; 0 when the geometry is not handled, else flags: 1 stepped, 2 F.illum \
        accumulated inside the step kernel, 4 F.inj applied inside the step kernel, 8 F.epi applied  \
        inside the step kernel */                                                                         \

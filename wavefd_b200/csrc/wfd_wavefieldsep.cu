@@ -18,8 +18,8 @@
 // length >= 4nz - 1 (Bluestein's algorithm, which any nz that is not a power of two needed). x and y
 // may differ by orders of magnitude (a saved V^2/B-scaled derivative against a pressure), and a
 // transform rounds relative to the larger of the two it carries, so each is first brought to a maximum
-// of about 1 by a power of two of its own: without that the result was 1.7e-6 off at 40:1, with it
-// MEASURED_ERR.
+// of about 1 by a power of two of its own: without that the result was 1.7e-6 off (relative L2
+// against float64) at 40:1, with it 1.8e-7 at any ratio (Bluestein transforms of each column: 3.3e-7).
 //
 // One thread holds 8 points of both transforms (u: odd cells, v: even cells), L/8 threads a column.
 // Stages are radix 8 (the last one 2 or 4 when log2 L is no multiple of 3), decimation in frequency
