@@ -428,7 +428,7 @@ void order_props_after(Batch *b) {
 
 int batch_sync(Batch *b) {
     if (int rc = bcheck(b, cudaStreamSynchronize(b->stream), "batch synchronize")) return rc;
-    if (wfd_fast::fused_status_and_clear() | wfd_strict::fused_status_and_clear())
+    if (wfd::take_status())
         return bfail(b, WFD_ERR_TIMEOUT, "a batched step kernel timed out waiting for its tile loads");
     return WFD_OK;
 }

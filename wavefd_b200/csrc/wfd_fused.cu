@@ -42,9 +42,4 @@ void fused_set_pipeline_wait(unsigned long long ns) {
     aniso3d_set_pipeline_wait(ns);
 }
 
-// timeout flags of every fused kernel, cleared on read
-unsigned fused_status_and_clear() {
-    return iso3d_status_and_clear() | aniso3d_status_and_clear() | vti3d_status_and_clear();
-}
-
 }  // namespace WFD_NS

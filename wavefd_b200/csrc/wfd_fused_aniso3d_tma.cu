@@ -65,8 +65,6 @@ static_assert((OFF_MAT * 4) % 128 == 0 && (M_STAGE * 4) % 128 == 0, "TMA alignme
 static_assert(OFF_BAR % 2 == 0, "mbarrier alignment");
 static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
 
-__device__ unsigned int d_status;
-
 __device__ __forceinline__ float2 ld2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
 __device__ __forceinline__ void st2(float *p, float2 v) { *reinterpret_cast<float2 *>(p) = v; }
 __device__ __forceinline__ float2 bc2(float s) { return make_float2(s, s); }
@@ -431,7 +429,7 @@ __global__ void __launch_bounds__(NT, 1)
             for (int rp = 0; rp < 8 && rp < nplanes; rp++) image_plane(rseq + rp);
         if (fail) {
             atomicExch(abort_flag, 1);
-            atomicOr(&d_status, 1u);
+            *(volatile unsigned *)F.status = 1u;
         }
         __syncthreads();
 
@@ -492,7 +490,7 @@ __global__ void __launch_bounds__(NT, 1)
             else ok_w = false;
             if (!ok_w) {
                 atomicExch(abort_flag, 1);
-                atomicOr(&d_status, 1u);
+                *(volatile unsigned *)F.status = 1u;
             }
             const float *ring[8];
             {
@@ -725,7 +723,7 @@ void aniso3d_tma_batch(const Grid &gc, int phys, const AnisoShotDesc *shots, con
                        int nitems, int *counter, int grid, cudaStream_t s) {
     if (phys == TTI) {
         aniso_grid_cap<TTI, false>();
-        k_aniso3d_tma<TTI, false, true><<<grid, NT, SMEM_BYTES, s>>>(gc, Fields{}, AnisoMaps{}, 0, 0, 0, 1, shots,
+        k_aniso3d_tma<TTI, false, true><<<grid, NT, SMEM_BYTES, s>>>(gc, batch_fields(), AnisoMaps{}, 0, 0, 0, 1, shots,
                                                                      sel, items, nitems, counter);
     } else {
         vti3d_tma_batch(gc, shots, sel, items, nitems, counter, grid, s);
@@ -735,13 +733,6 @@ void aniso3d_tma_batch(const Grid &gc, int phys, const AnisoShotDesc *shots, con
 void aniso3d_set_pipeline_wait(unsigned long long ns) {
     const uint64_t v = ns;
     cudaMemcpyToSymbol(wfd_dev::d_pipeline_wait_ns, &v, sizeof(v));
-}
-
-unsigned aniso3d_status_and_clear() {
-    unsigned v = 0, z = 0;
-    cudaMemcpyFromSymbol(&v, d_status, sizeof(v));
-    if (v) cudaMemcpyToSymbol(d_status, &z, sizeof(z));
-    return v;
 }
 
 }  // namespace WFD_NS

@@ -55,8 +55,6 @@ static_assert((STAGE * 4) % 128 == 0 && (S_BH * 4) % 128 == 0 && (S_PN * 4) % 12
 
 enum Mode { INNER = 0, EDGE = 1, TOP = 2 };
 
-__device__ unsigned int d_status;
-
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 __device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
 __device__ __forceinline__ float2 ld2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
@@ -529,7 +527,7 @@ __global__ void __launch_bounds__(NT, 3)
             const bool landed = mbar_wait(&bars[slot], par);
             if (!landed) {
                 atomicExch(abort_flag, 1);
-                atomicOr(&d_status, 1u);
+                *(volatile unsigned *)F.status = 1u;
             }
             // a group whose wait ran out may still be in flight: the drain below waits for it
             if (tid == 0 && landed) out_from = gs + 1;
@@ -664,20 +662,13 @@ bool iso3d_tma_describe(const Grid &g, const Fields &F, int xchunk, IsoShotDesc 
 
 void iso3d_tma_batch(const Grid &gc, const IsoShotDesc *shots, const int *sel, const int2 *items, int nitems,
                      int *counter, int grid, cudaStream_t s) {
-    k_iso3d_tma<true><<<grid, NT, SMEM_BYTES, s>>>(gc, Fields{}, IsoMaps{}, 0, 0, 0, 1, shots, sel, items, nitems,
+    k_iso3d_tma<true><<<grid, NT, SMEM_BYTES, s>>>(gc, batch_fields(), IsoMaps{}, 0, 0, 0, 1, shots, sel, items, nitems,
                                                    counter);
 }
 
 void iso3d_set_pipeline_wait(unsigned long long ns) {
     const uint64_t v = ns;
     cudaMemcpyToSymbol(wfd_dev::d_pipeline_wait_ns, &v, sizeof(v));
-}
-
-unsigned iso3d_status_and_clear() {
-    unsigned v = 0, z = 0;
-    cudaMemcpyFromSymbol(&v, d_status, sizeof(v));
-    if (v) cudaMemcpyToSymbol(d_status, &z, sizeof(z));
-    return v;
 }
 
 }  // namespace WFD_NS

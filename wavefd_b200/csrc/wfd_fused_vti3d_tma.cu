@@ -60,8 +60,6 @@ static_assert(OFF_BAR % 2 == 0, "mbarrier alignment");
 static_assert((STAGE * 4) % 128 == 0 && (PH_ * 4) % 128 == 0 && (MH_ * 4) % 128 == 0 && (OS * 4) % 128 == 0,
               "TMA destination alignment");
 
-__device__ unsigned int d_status;
-
 __device__ __forceinline__ float2 ld2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
 __device__ __forceinline__ void st2(float *p, float2 v) { *reinterpret_cast<float2 *>(p) = v; }
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
@@ -410,7 +408,7 @@ __global__ void __launch_bounds__(NT, 2)
             const bool landed = mbar_wait(&bars[gs % NS], (gs / NS) & 1u);
             if (!landed) {
                 atomicExch(abort_flag, 1);
-                atomicOr(&d_status, 1u);
+                *(volatile unsigned *)F.status = 1u;
             }
             // a group whose wait ran out may still be in flight: the drain below waits for it
             if (tid == ISSUER && landed) out_from = gs + 1;
@@ -616,20 +614,13 @@ bool vti3d_tma_describe(const Grid &g, const Fields &F, int xchunk, AnisoShotDes
 void vti3d_tma_batch(const Grid &gc, const AnisoShotDesc *shots, const int *sel, const int2 *items, int nitems,
                      int *counter, int grid, cudaStream_t s) {
     vti_grid_cap<false>();
-    k_vti3d_tma<false, true><<<grid, NT, SMEM_BYTES, s>>>(gc, Fields{}, AnisoMaps{}, 0, 0, 0, 1, shots, sel, items,
+    k_vti3d_tma<false, true><<<grid, NT, SMEM_BYTES, s>>>(gc, batch_fields(), AnisoMaps{}, 0, 0, 0, 1, shots, sel, items,
                                                          nitems, counter);
 }
 
 void vti3d_set_pipeline_wait(unsigned long long ns) {
     const uint64_t v = ns;
     cudaMemcpyToSymbol(wfd_dev::d_pipeline_wait_ns, &v, sizeof(v));
-}
-
-unsigned vti3d_status_and_clear() {
-    unsigned v = 0, z = 0;
-    cudaMemcpyFromSymbol(&v, d_status, sizeof(v));
-    if (v) cudaMemcpyToSymbol(d_status, &z, sizeof(z));
-    return v;
 }
 
 }  // namespace WFD_NS

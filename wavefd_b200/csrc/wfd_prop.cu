@@ -77,6 +77,24 @@ int prop_fail(Prop *p, int code, const std::string &msg) {
     return code;
 }
 
+unsigned *status_word() {
+    static unsigned *const word = [] {
+        void *p = nullptr;
+        if (cudaHostAlloc(&p, sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+            cudaGetLastError();
+            return (unsigned *)nullptr;
+        }
+        *(unsigned *)p = 0;
+        return (unsigned *)p;  // kept until the process ends: kernels of any object may write it
+    }();
+    return word;
+}
+
+bool take_status() {
+    unsigned *w = status_word();
+    return w && __atomic_exchange_n(w, 0u, __ATOMIC_ACQ_REL) != 0;
+}
+
 static int check_cuda(Prop *p, cudaError_t e, const char *what) {
     if (e == cudaSuccess) return WFD_OK;
     return prop_fail(p, WFD_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
@@ -126,6 +144,7 @@ Fields Prop::fields() const {
     F.mold = field[F_MOLD];
     F.mspace = field[F_MSPACE];
     F.illum = illum;
+    F.status = status_word();
     F.inj = inj;
     F.epi = epi;
     return F;
@@ -201,6 +220,7 @@ Prop *prop_create(int ndim, int phys, long fs, long nthread, long nx, long ny, l
         return nullptr;
     }
     p->own_stream = true;
+    status_word();  // allocated here, not by a step that may be under capture
     for (int f = 0; f < F_COUNT; f++) {
         if (!p->alloc[f]) continue;
 #if CUDART_VERSION >= 13000
@@ -310,8 +330,8 @@ void prop_setup_q(Prop *p, float freqQ, float qMin, float qInterior) {
 // ---------------------------------------------------------------------------------------------
 int prop_sync(Prop *p) {
     if (int rc = check_cuda(p, cudaStreamSynchronize(p->stream), "synchronize")) return rc;
-    // device status words of the TMA kernels: a bounded wait that ran out
-    if (wfd_fast::fused_status_and_clear() | wfd_strict::fused_status_and_clear())
+    // the TMA kernels' status word: a bounded wait that ran out
+    if (take_status())
         return prop_fail(p, WFD_ERR_TIMEOUT, "a fused step kernel timed out waiting for its tile loads");
     return WFD_OK;
 }
@@ -319,6 +339,7 @@ int prop_sync(Prop *p) {
 int prop_step(Prop *p, bool linear, bool sync) {
     Grid g = p->grid();
     Fields F = p->fields();
+    if (!F.status) return prop_fail(p, WFD_ERR_ALLOC, "status word allocation failed");
     // the step kernels read the epilogue's arrays 16 (Iso) or 8 bytes at a time: arrays at other
     // alignments take the separate kernels after the step
     auto a16 = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };

@@ -157,13 +157,14 @@ struct CachedTable {
     std::vector<PointsT<T>> raw;       // the caller's points, partition by partition
     std::vector<long> counts;          // points per partition
     unsigned long long last_use = 0;
-    T *d_dst = nullptr, *d_src = nullptr;  // device staging (groups, points)
-    T *h_dst = nullptr, *h_src = nullptr;  // pinned host staging
+    T *d_src = nullptr;                    // device staging (points)
+    T *h_dst = nullptr, *h_src = nullptr;  // pinned host staging (groups, points), mapped
 };
 
 // Host loops over the points of a drop-in call use up to the caller's thread count (the reference's
 // nthreads argument) once they are long enough to pay for it.
 constexpr long kParallelPoints = 8192;
+constexpr long kMappedPoints = 4096;
 
 template <class T>
 bool same_points(const CachedTable<T> &e, int by_receiver, void **partitions, size_t npartitions,
@@ -188,7 +189,6 @@ bool same_points(const CachedTable<T> &e, int by_receiver, void **partitions, si
 template <class T>
 void free_entry(CachedTable<T> *e, cudaStream_t s) {
     release(e->t, s);
-    if (e->d_dst) cudaFreeAsync(e->d_dst, s);
     if (e->d_src) cudaFreeAsync(e->d_src, s);
     cudaStreamSynchronize(s);
     if (e->h_dst) cudaFreeHost(e->h_dst);
@@ -225,7 +225,6 @@ CachedTable<T> *lookup(TableCache<T> &cache, int by_receiver, void **partitions,
     build(e->t, e->raw, by_receiver);
     const size_t ng = (size_t)e->t.ngroups, np = (size_t)e->t.npoints;
     bool ok = upload(e->t, s);
-    ok = ok && wfd::dMallocAsync(&e->d_dst, sizeof(T) * (ng + 1), s) == cudaSuccess;
     ok = ok && wfd::dMallocAsync(&e->d_src, sizeof(T) * (np + 1), s) == cudaSuccess;
     ok = ok && wfd::dMallocHost(&e->h_dst, sizeof(T) * (ng + 1)) == cudaSuccess;
     ok = ok && wfd::dMallocHost(&e->h_src, sizeof(T) * (np + 1)) == cudaSuccess;
@@ -269,22 +268,24 @@ void dropin(int by_receiver, T *dst, long dst_stride, long dst_off, const T *src
     const bool dst_dev = device_accessible(dst);
     const bool src_dev = device_accessible(src);
     const long ng = t.ngroups, np = t.npoints;
+    // The kernel reads and writes the pinned staging itself: each written location once and coalesced, and
+    // up to kMappedPoints values read by one thread per group. More go through the device (a copy's
+    // fixed cost, about 10 us with its wait, is then less than the scattered reads).
+    const bool copy = np > kMappedPoints;
     if (!src_dev) {
 #pragma omp parallel for num_threads(nth) if (np >= kParallelPoints) schedule(static)
         for (long j = 0; j < np; j++) e->h_src[j] = src[t.other[j] * src_stride + src_off];
-        cudaMemcpyAsync(e->d_src, e->h_src, sizeof(T) * (size_t)np, cudaMemcpyHostToDevice, s);
+        if (copy) cudaMemcpyAsync(e->d_src, e->h_src, sizeof(T) * (size_t)np, cudaMemcpyHostToDevice, s);
     }
     if (!dst_dev) {
 #pragma omp parallel for num_threads(nth) if (ng >= kParallelPoints) schedule(static)
         for (long g = 0; g < ng; g++) e->h_dst[g] = dst[t.key[g] * dst_stride + dst_off];
-        cudaMemcpyAsync(e->d_dst, e->h_dst, sizeof(T) * (size_t)ng, cudaMemcpyHostToDevice, s);
     }
     k_scatter_groups<T><<<nb(ng), 256, 0, s>>>(ng, t.d_key, t.d_start, t.d_other, t.d_c,
-                                               dst_dev ? dst : e->d_dst, dst_dev ? dst_stride : 0,
+                                               dst_dev ? dst : e->h_dst, dst_dev ? dst_stride : 0,
                                                dst_dev ? dst_off : 0, dst_dev ? 0 : 1,
-                                               src_dev ? src : e->d_src, src_dev ? src_stride : 0,
+                                               src_dev ? src : (copy ? e->d_src : e->h_src), src_dev ? src_stride : 0,
                                                src_dev ? src_off : 0, src_dev ? 0 : 1);
-    if (!dst_dev) cudaMemcpyAsync(e->h_dst, e->d_dst, sizeof(T) * (size_t)ng, cudaMemcpyDeviceToHost, s);
     cudaError_t err = cudaStreamSynchronize(s);
     if (err != cudaSuccess) {
         set_global_error(WFD_ERR_CUDA, cudaGetErrorString(err));

@@ -14,6 +14,7 @@ weights agree to rounding, not bit for bit; the GPU consumes whatever table it i
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import numpy as np
 
@@ -192,21 +193,30 @@ def receiver_blocking(points, nthreads=8):
     return blocking(points, "ir", nthreads)
 
 
+_PartPtr = ctypes.POINTER(ctypes.POINTER(SourcePoint32))
+_FloatPtr = ctypes.POINTER(ctypes.c_float)
+
+
 def _partition_args(partitions):
-    ptrs = (ctypes.POINTER(SourcePoint32) * len(partitions))(
-        *[p.ctypes.data_as(ctypes.POINTER(SourcePoint32)) for p in partitions])
+    ptrs = (ctypes.c_void_p * len(partitions))(*[p.ctypes.data for p in partitions])
     counts = (ctypes.c_long * len(partitions))(*[len(p) for p in partitions])
-    return ptrs, counts
+    return ctypes.cast(ptrs, _PartPtr), counts
 
 
 def _fp(a):
-    return a.ctypes.data_as(ctypes.POINTER(ctypes.c_float))
+    return a.ctypes.data_as(_FloatPtr)
+
+
+@functools.lru_cache(maxsize=8)
+def _abi(lib):
+    """The declared exports of a library (a time loop calls them twice a step)."""
+    return SpacetimeABI(lib)
 
 
 def injectdata(field, partitions, data, it, nthreads=8, lib=None):
     """field[iu] += c * data[it, ir] (1-based it; data shaped (ntraces, nt) C order = Julia (nt, ntraces))."""
     from . import _lib
-    st = SpacetimeABI(lib or _lib.library())
+    st = _abi(lib or _lib.library())
     ptrs, counts = _partition_args(partitions)
     nt = data.shape[-1]
     st.injectdata_float(_fp(field), _fp(data), it, nt, ptrs, len(partitions), counts, nthreads)
@@ -214,7 +224,7 @@ def injectdata(field, partitions, data, it, nthreads=8, lib=None):
 
 def extractdata(data, field, it, partitions, nthreads=8, lib=None):
     from . import _lib
-    st = SpacetimeABI(lib or _lib.library())
+    st = _abi(lib or _lib.library())
     ptrs, counts = _partition_args(partitions)
     nt = data.shape[-1]
     st.extractdata_float(_fp(data), _fp(field), ptrs, len(partitions), counts, it, nt, nthreads)
