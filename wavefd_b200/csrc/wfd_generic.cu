@@ -484,7 +484,12 @@ __global__ void __launch_bounds__(kThreads) k_image_iso_b(Grid g, int which, Fie
 }
 
 // Born VEA, first launch: the gradient triples of P and M and the sandwich into tp2, tm2 (3D VTI
-// .h:480-511; 3D TTI .h:481-512; 2D alike)
+// .h:480-511; 3D TTI .h:481-512; 2D alike). TTI, fast build: the vectors are rotated back to the grid's axes
+// here, once a cell, and the second launch is the plain divergence: the rotated D- is a sum over the
+// components of derivatives of (weight x component), each weight taken at the tap's own cell, so that
+// the sum over components can come first (3 derivatives a vector instead of 8, and none of their weights'
+// loads; the strict build keeps the reference's order). 200 x 180 x 240: 1009 -> 373 us for the call (the
+// marching kernels of wfd_pass3d.cu given the same algebra took 356 us, and more than these in VTI and Iso).
 template <bool ROT>
 __global__ void __launch_bounds__(kThreads) k_born_vea_1(Grid g, Fields F, const float *__restrict__ de,
                                                          const float *__restrict__ da, const float *__restrict__ P,
@@ -498,6 +503,26 @@ __global__ void __launch_bounds__(kThreads) k_born_vea_1(Grid g, Fields F, const
     grad_at<ROT>(g, F, P, k, z, r, tp1);
     grad_at<ROT>(g, F, M, k, z, r, tm1);
     const float A = F.eta[k], B = F.b[k], Fv = F.f[k], dE = de[k], dA = da[k];
+#if !WFD_STRICT
+    if (ROT) {
+        const float e = +2 * B * dE, w = 2 * B * Fv * A * dA, X = dA * B * Fv * (1 - 2 * A * A) / sqrtf(1 - A * A);
+        const float t1 = e * tp1[0], t2 = e * tp1[1], t3 = X * tm1[2] - w * tp1[2], m3 = w * tm1[2] + X * tp1[2];
+        const float st = F.st[k], ct = F.ct[k];
+        if (g.ndim == 3) {
+            const float sp = F.sp[k], cp = F.cp[k];
+            tp2.p[0][k] = ct * cp * t1 - sp * t2 + st * cp * t3;
+            tp2.p[1][k] = ct * sp * t1 + cp * t2 + st * sp * t3;
+            tm2.p[0][k] = st * cp * m3;
+            tm2.p[1][k] = st * sp * m3;
+        } else {
+            tp2.p[0][k] = ct * t1 + st * t3;
+            tm2.p[0][k] = st * m3;
+        }
+        tp2.p[2][k] = ct * t3 - st * t1;
+        tm2.p[2][k] = ct * m3;
+        return;
+    }
+#endif
     tp2.p[0][k] = (+2 * B * dE) * tp1[0];
     if (g.ndim == 3) tp2.p[1][k] = (+2 * B * dE) * tp1[1];
     tp2.p[2][k] = (-2 * B * Fv * A * dA) * tp1[2] + (dA * B * Fv * (1 - 2 * A * A) / sqrtf(1 - A * A)) * tm1[2];
@@ -518,8 +543,9 @@ __global__ void __launch_bounds__(kThreads) k_born_vea_2(Grid g, Fields F, const
     cell_xyz(g, k, x, y, z);
     const int r = region(g, x, y, z);
     float lp[3], lm[3];
-    dminus_at<ROT>(g, F, tp2.p[0], tp2.p[1], tp2.p[2], k, z, r, lp);
-    dminus_at<ROT>(g, F, tm2.p[0], tm2.p[1], tm2.p[2], k, z, r, lm);
+    constexpr bool BACK = ROT && WFD_STRICT;  // (the fast build's first launch rotated back)
+    dminus_at<BACK>(g, F, tp2.p[0], tp2.p[1], tp2.p[2], k, z, r, lp);
+    dminus_at<BACK>(g, F, tm2.p[0], tm2.p[1], tm2.p[2], k, z, r, lm);
     const float V = F.v[k], B = F.b[k], dV = dv[k];
     const float dt2v2OverB = g.dt * g.dt * V * V / B;
     const float factor = 2 * B * dV / (V * V * V);
