@@ -32,7 +32,7 @@ FAST = ["-DWFD_STRICT=0", "-fmad=true", "-prec-div=false", "-prec-sqrt=false", "
 HOST = ["-Xcompiler", "-fopenmp"]  # host loops of the drop-in calls use the caller's thread count
 
 KERNEL_SOURCES = ["wfd_generic.cu", "wfd_pass3d.cu", "wfd_fused.cu", "wfd_fused_iso3d_tma.cu",
-                  "wfd_fused_aniso3d_tma.cu", "wfd_fused_vti3d_tma.cu", "wfd_fused_iso2d.cu", "wfd_fused_aniso2d.cu",
+                  "wfd_fused_aniso3d_tma.cu", "wfd_fused_vti3d_tma.cu", "wfd_loop2d.cu", "wfd_fused_iso2d.cu", "wfd_fused_aniso2d.cu",
                   "wfd_wavefieldsep.cu"]
 HOST_SOURCES = ["wfd_prop.cu", "wfd_bornimage.cu", "wfd_capi.cu", "wfd_addon.cu", "wfd_spacetime.cu",
                 "wfd_tma_host.cu", "wfd_noalloc.cu", "wfd_batch.cu", "wfd_codec.cu", "wfd_interp.cu", "wfd_illum.cu", "wfd_snapio.cu"]

@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(NT) k_aniso2d_fused(Grid g, Fields F) {
 // every tile's step with its source injection (CTAs take turns over the tiles; with as many CTAs as
 // tiles each keeps its tile and its material boxes), a grid-wide barrier, then the receiver
 // extraction from the new pCur; the pointer swaps of every step are the alternation of the two
-// arrays of each field.
+// arrays of each field. (Fast build: only with a CTA per tile; larger grids take wfd_loop2d.cu.)
 template <int PHYS>
 __global__ void __launch_bounds__(NT) k_aniso2d_run(Grid g, Fields F, long nsteps, long it0, RunExtract ex,
                                                     unsigned *sync_words) {
@@ -328,6 +328,9 @@ int aniso2d_run(const Grid &g, int phys, const Fields &F, long nsteps, long it0,
     }
     if (cap[which] <= 0) return -1;
     const long ntiles = ((g.nz + TZ - 1) / TZ) * ((g.nx + TX - 1) / TX);
+#if !WFD_STRICT
+    if (ntiles > cap[which]) return -1;  // wfd_loop2d.cu takes those
+#endif
     const int grid = (int)(ntiles < cap[which] ? ntiles : cap[which]);
     Grid gg = g;
     Fields FF = F;
@@ -337,7 +340,6 @@ int aniso2d_run(const Grid &g, int phys, const Fields &F, long nsteps, long it0,
     void *args[] = {&gg, &FF, &ns, &i0, &ee, &sw};
     return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(NT), args, SMEM_BYTES, s) == cudaSuccess ? 0 : 1;
 }
-
 bool fused_aniso2d(const Grid &g, int phys, int linear, const Fields &F, cudaStream_t s) {
     if (g.ndim != 2) return false;
     if (phys == VTI) return linear ? launch2<VTI, true>(g, F, s) : launch2<VTI, false>(g, F, s);

@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(NT) k_iso2d_fused(Grid g, Fields F) {
     tile_step(g, F, (long)blockIdx.y * TX, (long)blockIdx.x * TZ, it, sm);
 }
 
+#if WFD_STRICT  // (the fast build: wfd_loop2d.cu)
 // A whole time loop in one launch: nsteps steps, each followed by its source injection (in the step,
 // per tile) and, after a grid-wide barrier, its receiver extraction from the new field, at time
 // indices it0, it0+1, ...; the pointer swap of every step is the alternation of F.pcur and F.pold.
@@ -256,6 +257,8 @@ __global__ void __launch_bounds__(NT) k_iso2d_run(Grid g, Fields F, long nsteps,
         }
     }
 }
+#endif
+
 // The whole time loop with every tile resident in one CTA (as many CTAs as tiles, all co-resident).
 // B stays in shared memory and V, Q and the tile's pOld in registers; the pCur box keeps the tile's
 // own cells from the step before (its new field), so that a step reloads only the box's ring (the
@@ -465,14 +468,16 @@ __global__ void __launch_bounds__(NT, 2) k_iso2d_run_res(Grid g, Fields F, long 
 int iso2d_run(const Grid &g, const Fields &F, long nsteps, long it0, const RunExtract &ex, unsigned *sync_words,
               cudaStream_t s) {
     if (g.ndim != 2) return -1;
-    // co-resident CTAs of the two forms (0: the device has no cooperative launch)
+    // co-resident CTAs of the two forms (0: no cooperative launch, or the form is not in this build)
     static int cap = -1, cap_res = 0;
     if (cap < 0) {
         int dev = 0, sms = 0, per = 0, per_res = 0, coop = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+#if WFD_STRICT
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_iso2d_run, NT, 0);
+#endif
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_res, k_iso2d_run_res, NT, 0);
         cap = coop ? sms * per : 0;
         cap_res = coop ? sms * per_res : 0;
@@ -487,7 +492,10 @@ int iso2d_run(const Grid &g, const Fields &F, long nsteps, long it0, const RunEx
     RunExtract ee = ex;
     unsigned *sw = sync_words;
     void *args[] = {&gg, &FF, &ns, &i0, &ee, &sw};
-    const void *fn = resident ? (const void *)k_iso2d_run_res : (const void *)k_iso2d_run;
+    const void *fn = (const void *)k_iso2d_run_res;
+#if WFD_STRICT
+    if (!resident) fn = (const void *)k_iso2d_run;
+#endif
     return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(NT), args, 0, s) == cudaSuccess ? 0 : 1;
 }
 

@@ -147,6 +147,9 @@ struct TileInfo {
     /* 3D Iso: 0 not handled, 1 stepped (ragged rows: F.illum and F.epi not applied), 2 stepped with     \
        F.illum and F.epi */                                                                              \
     int fused_iso3d_tma(const wfd::Grid &g, const wfd::Fields &F, cudaStream_t s);                       \
+    /* a 2D loop as two passes a step with a barrier between (fast build only; S: 2 or 4 scratch arrays) */ \
+    int loop2d_run(const wfd::Grid &g, int phys, const wfd::Fields &F, const wfd::Scratch &S, long nsteps, \
+                   long it0, const wfd::RunExtract &ex, unsigned *sync_words, cudaStream_t s);           \
     bool fused_aniso3d_tma(const wfd::Grid &g, int phys, int linear, const wfd::Fields &F, cudaStream_t s); \
     bool fused_vti3d_tma(const wfd::Grid &g, int linear, const wfd::Fields &F, cudaStream_t s);         \
     bool vti3d_tma_describe(const wfd::Grid &g, const wfd::Fields &F, int xchunk, wfd::AnisoShotDesc *d, \

@@ -459,13 +459,15 @@ extern "C" int WFD_Prop_Run(void *prop, long nsteps, long it0, void *src_table, 
             ex = wfd::RunExtract{rec->t.ngroups, rec->t.d_key, rec->t.d_start, rec->t.d_other, rec->t.d_c, traces, nt};
         unsigned *words = reinterpret_cast<unsigned *>(d_it + 2);
         const wfd::Grid g = p->grid();
-        int r;
+        int r = -1;
         if (p->phys == wfd::ISO)
             r = p->strict ? wfd_strict::iso2d_run(g, F, nsteps, it0, ex, words, s)
-                          : wfd_fast::iso2d_run(g, F, nsteps, it0, ex, words, s);
+                          : wfd_fast::iso2d_run(g, F, nsteps, it0, ex, words, s);  // tiles all resident, or -1
         else
             r = p->strict ? wfd_strict::aniso2d_run(g, p->phys, F, nsteps, it0, ex, words, s)
-                          : wfd_fast::aniso2d_run(g, p->phys, F, nsteps, it0, ex, words, s);
+                          : wfd_fast::aniso2d_run(g, p->phys, F, nsteps, it0, ex, words, s);  // the same
+        if (r < 0 && !p->strict)
+            r = wfd_fast::loop2d_run(g, p->phys, F, p->scratch(), nsteps, it0, ex, words, s);
         if (r == 0) {
             unsigned status = 0;
             cudaMemcpyAsync(&status, words + 2, sizeof status, cudaMemcpyDeviceToHost, s);
