@@ -17,10 +17,14 @@
 // applied as selects on values computed everywhere; three code variants: interior tiles (no
 // selects), edge tiles (selects), and the top tile with a free surface (selects plus the image
 // stencils above kz = 0, which only the first z quad needs).
-// Persistent CTAs loop over (tile, x-chunk) items; a chunk starts with 14 warm-up planes that only
-// fill the queues. With an illumination sum attached (single objects), each cell's pCur^2 is added
-// to it as the cell is updated. Waits are bounded; on timeout the kernel records an error in a device status
-// word and leaves. Requires nz % 4 == 0 (TMA row pitch); the caller falls back otherwise.
+// Persistent CTAs loop over (tile, x-chunk) items; a chunk starts by filling its queues from global memory in
+// one go (all of its loads in flight together) and only then asks for its first groups. 14 warm-up planes
+// through the pipeline, each a wait for a whole group, took 5.1 us more a chunk, and so kept chunks above 16
+// planes and small grids on few CTAs: with the fill a chunk costs about 2 planes and may be 2 planes long.
+// Measured, us a step before and now: 40^3 21.6, 8.2; 64x60x68 26.6, 10.3; 128^3 33.6, 23.7; 300x200x248 139.6,
+// 133.3; 512^3 970, 955. With an illumination sum attached (single objects), each cell's pCur^2 is added
+// to it as the cell is updated. Waits are bounded; on timeout the kernel records an error in the object's
+// status word and leaves. Rows that TMA cannot address (nz % 4 != 0) are staged by cp.async instead.
 #include "wfd_kernels.h"
 #include "wfd_ragged.cuh"
 #include "wfd_tma.cuh"
@@ -45,7 +49,7 @@ constexpr int TZW = TZ + 8;  // pass-1 z output columns z0-4 .. z0+35 (39 used)
 constexpr int S_PH = 0, S_BH = S_PH + PH_, S_PN = S_BH + BH_, S_BN = S_PN + OS, S_PO = S_BN + OS, S_V = S_PO + OS,
               S_Q = S_V + OS, STAGE = S_Q + OS;
 constexpr unsigned GROUP_BYTES = 4u * STAGE;
-constexpr int WARMUP = 14;
+constexpr int START = 2;  // a chunk's start in planes, for the work split
 constexpr int OFF_TY = NS * STAGE;
 constexpr int OFF_TZ = OFF_TY + TYR * TZ;
 constexpr int OFF_BAR = OFF_TZ + TY * TZW;
@@ -406,6 +410,7 @@ __global__ void __launch_bounds__(NT, 3)
         Grid g = g0;
         const CUtensorMap *maps = M.m;
         float *out_pold = F.pold, *out_pspace = F.pspace;
+        const float *in_p = F.pcur, *in_b = F.b;
         int ntz = ntz0, nty = nty0, xchunk = xchunk0;
         long w = wstat;
         if (BATCH) {
@@ -425,6 +430,8 @@ __global__ void __launch_bounds__(NT, 3)
             maps = d->m;
             out_pold = d->pold;
             out_pspace = d->pspace;
+            in_p = d->pcur;
+            in_b = d->b;
             ntz = d->ntz;
             nty = d->nty;
             xchunk = d->xchunk;
@@ -444,8 +451,7 @@ __global__ void __launch_bounds__(NT, 3)
         const bool own = z < g.nz && y < g.ny;
         const long xbeg = (long)chi * xchunk;
         const long xend = xbeg + xchunk < g.nx ? xbeg + xchunk : g.nx;
-        const long jstart = xbeg - WARMUP;
-        const int ngroups = (int)(xend - jstart);
+        const int ngroups = (int)(xend - xbeg);
         const bool tile_top = z0 == 0 && g.fs;
         unsigned txmask = 0;  // cells of this thread whose pass-1 x output is computed (given x)
         unsigned fmask = 0;   // cells of this thread that are updated (given x)
@@ -467,14 +473,12 @@ __global__ void __launch_bounds__(NT, 3)
                 auto plane = [&](const float *f, long x) { return f + min(max(x, 0l), g.nx - 1) * g.sx; };
                 BoxT::load(s + S_PN, plane(F.pcur, jj + 7), z0, y0, nz, warp, lane);
                 BoxT::load(s + S_BN, plane(F.b, jj + 3), z0, y0, nz, warp, lane);
-                if (jj >= xbeg) {  // the warm-up planes only fill the queues
-                    const long k = jj * g.sx;
-                    BoxP::load(s + S_PH, F.pcur + k, z0 - 8, y0 - 7, nz, warp, lane);
-                    BoxB::load(s + S_BH, F.b + k, z0 - 4, y0 - 4, nz, warp, lane);
-                    BoxT::load(s + S_PO, out_pold + k, z0, y0, nz, warp, lane);
-                    BoxT::load(s + S_V, F.v + k, z0, y0, nz, warp, lane);
-                    BoxT::load(s + S_Q, F.q + k, z0, y0, nz, warp, lane);
-                }
+                const long k = jj * g.sx;
+                BoxP::load(s + S_PH, F.pcur + k, z0 - 8, y0 - 7, nz, warp, lane);
+                BoxB::load(s + S_BH, F.b + k, z0 - 4, y0 - 4, nz, warp, lane);
+                BoxT::load(s + S_PO, out_pold + k, z0, y0, nz, warp, lane);
+                BoxT::load(s + S_V, F.v + k, z0, y0, nz, warp, lane);
+                BoxT::load(s + S_Q, F.q + k, z0, y0, nz, warp, lane);
                 cp_async_arrive(bar);
                 return;
             }
@@ -487,11 +491,6 @@ __global__ void __launch_bounds__(NT, 3)
             tma_load_3d(s + S_V, mV, bar, z0, y0, (int)jj);
             tma_load_3d(s + S_Q, mQ, bar, z0, y0, (int)jj);
         };
-        if (RAG || tid == 0) {
-            for (int q = 0; q < D && q < ngroups; q++) issue(jstart + q, gseq + q);
-            out_from = gseq;
-            out_to = gseq + (D < ngroups ? D : ngroups);
-        }
         // queues: qp[(q+i)&7] = pCur(j+i), qt[(q+i)&7] = pass-1 x output at plane j-4+i
         float2 qp[8][2], qt[8][2];
 #pragma unroll
@@ -501,11 +500,41 @@ __global__ void __launch_bounds__(NT, 3)
                 qp[i][h] = bc2(0.0f);
                 qt[i][h] = bc2(0.0f);
             }
+        // at the chunk's first plane: qp[i] = pCur(xbeg+i), qt[i] the output at plane xbeg-4+i, i = 0..6, from
+        // planes xbeg-7 .. xbeg+6 (those outside the grid feed only outputs that are zero, and read the
+        // nearest plane)
+        if (own) {
+            const long kc = (long)y * g.nz + z;
+            auto at = [&](const float *p, long x, int h) {
+                const float *q = p + min(max(x, 0l), g.nx - 1) * g.sx + kc + 2 * h;
+                return RAG ? make_float2(__ldg(q), __ldg(q + 1)) : __ldg(reinterpret_cast<const float2 *>(q));
+            };
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                float2 w[14], b[7];
+#pragma unroll
+                for (int i = 0; i < 14; i++) w[i] = at(in_p, xbeg - 7 + i, h);
+#pragma unroll
+                for (int i = 0; i < 7; i++) b[i] = at(in_b, xbeg - 4 + i, h);
+#pragma unroll
+                for (int i = 0; i < 7; i++) {
+                    const bool xin = xbeg - 4 + i >= 4 && xbeg - 4 + i < g.nx - 4;
+                    const float2 s = st8p(g, w[i], w[i + 1], w[i + 2], w[i + 3], w[i + 4], w[i + 5], w[i + 6], w[i + 7]);
+                    qt[i][h] = keep2(xin ? txmask : 0u, 2 * h, mul2(b[i], mul2(bc2(g.idx), s)), bc2(0.0f));
+                    qp[i][h] = w[7 + i];
+                }
+            }
+        }
+        if (RAG || tid == 0) {
+            for (int q = 0; q < D && q < ngroups; q++) issue(xbeg + q, gseq + q);
+            out_from = gseq;
+            out_to = gseq + (D < ngroups ? D : ngroups);
+        }
         unsigned slot = gseq % NS, par = (gseq / NS) & 1u;  // stage and phase of group gseq + q
 
         bool stop = false;
         for (int q = 0; q < ngroups; q++) {
-            const long j = jstart + q;
+            const long j = xbeg + q;
             const unsigned gs = gseq + q;
             if ((RAG || tid == 0) && q + D < ngroups) {
                 issue(j + D, gs + D);
@@ -514,7 +543,7 @@ __global__ void __launch_bounds__(NT, 3)
             // the epilogue's inputs of plane j, loaded now so that their latency hides behind the wait
             // and the queue work (born: dV, DP; imaging: the image, DP)
             float4 ea = make_float4(0.0f, 0.0f, 0.0f, 0.0f), eb = ea;
-            if (EPI && own && j >= xbeg) {
+            if (EPI && own) {
                 const long k = j * g.sx + (long)y * g.nz + z;
                 if (F.epi.born_dv) {
                     ea = __ldg(reinterpret_cast<const float4 *>(F.epi.born_dv + k));
@@ -551,7 +580,7 @@ __global__ void __launch_bounds__(NT, 3)
                     default: queue_phase<7>(qp, qt, g, xin_a, txmask, pn, bn, sx, pc); break;
                 }
             }
-            if (j >= xbeg) {
+            {
                 const bool xin = j >= 4 && j < g.nx - 4;
                 // one code path for every tile (the selects are cheap, code size is not)
                 ext_stage<EDGE>(g, xin, tile_top, z0, emask, st, TYs, TZs);
@@ -614,15 +643,15 @@ int fused_iso3d_tma(const Grid &g, const Fields &F, cudaStream_t s) {
     const int grid_cap = iso_grid_cap();
     const int ntz = (int)((g.nz + TZ - 1) / TZ);
     const int nty = (int)((g.ny + TY - 1) / TY);
-    // x-chunking: balance the last wave of persistent CTAs against the warm-up planes per chunk
+    // x-chunking: balance the last wave of persistent CTAs against the start of each chunk
     const long tiles = (long)ntz * nty;
     int best_nch = 1;
     double best_cost = 1e30;
-    for (int nch = 1; nch <= 64 && nch <= g.nx / 16 + 1; nch++) {
+    for (int nch = 1; nch <= 64 && nch <= g.nx / 2 + 1; nch++) {
         const long chunk = (g.nx + nch - 1) / nch;
         const long items = tiles * nch;
         const double waves = (double)((items + grid_cap - 1) / grid_cap);
-        const double cost = waves * (double)(chunk + WARMUP * 0.35);
+        const double cost = waves * (chunk + START);
         if (cost < best_cost) {
             best_cost = cost;
             best_nch = nch;
@@ -644,6 +673,8 @@ bool iso3d_tma_describe(const Grid &g, const Fields &F, int xchunk, IsoShotDesc 
         if (!iso_maps(g, F, d->m)) return false;
         d->pold = F.pold;
         d->pspace = F.pspace;
+        d->pcur = F.pcur;
+        d->b = F.b;
         d->nx = (int)g.nx;
         d->ny = (int)g.ny;
         d->nz = (int)g.nz;
@@ -654,7 +685,7 @@ bool iso3d_tma_describe(const Grid &g, const Fields &F, int xchunk, IsoShotDesc 
     if (t) {
         t->tz = TZ;
         t->ty = TY;
-        t->warmup = WARMUP;
+        t->warmup = START;
         t->grid_cap = iso_grid_cap();
     }
     return true;

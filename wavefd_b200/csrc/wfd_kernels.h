@@ -90,6 +90,7 @@ struct AnisoMaps {
 struct alignas(64) IsoShotDesc {
     CUtensorMap m[7];
     float *pold, *pspace;
+    const float *pcur, *b;  // read directly by a chunk's start
     int nx, ny, nz, ntz, nty, xchunk;
 };
 struct alignas(64) AnisoShotDesc {
@@ -101,7 +102,7 @@ struct alignas(64) AnisoShotDesc {
 // Tile geometry and capacity of a TMA step kernel, for the batch planner.
 struct TileInfo {
     int tz, ty;      // (z, y) cross-section of a tile
-    int warmup;      // planes swept before the first output plane of an x-chunk
+    int warmup;      // what an x-chunk's start costs, in planes
     int grid_cap;    // resident CTAs on this device (SMs x CTAs per SM)
 };
 
