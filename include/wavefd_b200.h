@@ -290,7 +290,7 @@ const char *WFD_Prop_Message(void *p);
 
 /* Failure-detection hook (no counterpart in the reference): the limit, in ns, of the waits of the TMA
  * step kernels for their tile loads (default 2 s; 0 restores it). A wait that runs out makes the
- * kernel record a timeout in its device status word, let its copies in flight land and leave; the
+ * kernel record a timeout in the object's status word, let its copies in flight land and leave; the
  * object then reports WFD_ERR_TIMEOUT. Tests shorten the limit to make a wait run out. Device-wide
  * and synchronous; not for use while other work runs. */
 int WFD_Debug_SetPipelineWait(unsigned long long ns);

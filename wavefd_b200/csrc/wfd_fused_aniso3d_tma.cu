@@ -24,7 +24,7 @@
 // kz = 0 into each ring plane of the top tile, the symmetric image of the z outputs into the halo
 // columns of the top tile. With an illumination sum attached (single objects), each cell's pCur^2
 // is added to it as the cell is updated. Waits are bounded; on timeout the kernel records an error
-// in a device status word and leaves. Requires nz % 4 == 0 (TMA row pitch).
+// in the object's status word and leaves. Requires nz % 4 == 0 (TMA row pitch).
 #include "wfd_kernels.h"
 #include "wfd_tma.cuh"
 

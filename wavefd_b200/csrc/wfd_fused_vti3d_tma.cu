@@ -21,7 +21,7 @@
 // images (antisymmetric pCur/mCur above kz = 0 in the z derivative, symmetric z outputs in D-) only
 // in the top tile. Persistent CTAs loop over (tile, x-chunk) items; chunks start with 14 warm-up
 // planes that only fill the queues (their groups load the queue boxes alone). Waits are bounded;
-// on timeout the kernel records an error in a device status word and leaves. With an illumination
+// on timeout the kernel records an error in the object's status word and leaves. With an illumination
 // sum attached (single objects), each cell's pCur^2 is added to it as the cell is updated.
 // Requires nz % 4 == 0.
 #include "wfd_kernels.h"

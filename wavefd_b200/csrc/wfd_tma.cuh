@@ -2,7 +2,7 @@
 //
 // Loads are tiled 3D tensor copies global -> shared, completed on an mbarrier with a transaction
 // count; no multicast. Every wait is bounded by the global timer: on timeout the caller records
-// an error in a device status word and leaves its loop instead of spinning forever.
+// an error in the object's status word and leaves its loop instead of spinning forever.
 #pragma once
 
 #include <cuda.h>
