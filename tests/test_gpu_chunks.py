@@ -25,7 +25,7 @@ def oracle():
     return Oracle()
 
 
-@pytest.mark.parametrize("physics", ["iso"])
+@pytest.mark.parametrize("physics", ["iso", "tti"])
 @pytest.mark.parametrize("shape", SHAPES)
 @pytest.mark.parametrize("fs", [True, False])
 def test_short_chunks(lib, oracle, physics, shape, fs):
