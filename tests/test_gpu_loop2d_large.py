@@ -1,0 +1,63 @@
+"""Whole 2D time loops on grids with more 64 x 16 tiles than any co-resident set of CTAs of 512 threads (four an
+SM), which the fast build runs as two passes a step (k_loop2d)."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+NT = 13
+
+
+def _run(physics, shape, fs, spts, rpts, loop=True):
+    """Fields and traces after NT steps, by one WFD_Prop_Run or by the stepping calls."""
+    import torch
+    from tests.harness import ABIRunner, make_model
+    from wavefd_b200 import _lib
+    from wavefd_b200.abi import SourcePoint32
+    lib = _lib.library()
+    nx, nz = shape
+    assert -(-nx // 16) * -(-nz // 64) > 4 * torch.cuda.get_device_properties(0).multi_processor_count
+    g = ABIRunner(lib, f"Prop2DAco{physics}DenQ_DEO2_FDTD", (nz, 1, nx), fs=fs)
+    g.load(make_model(2, physics.lower(), (nz, 1, nx), seed=8))
+    wav = torch.from_numpy(np.random.default_rng(4).standard_normal((2, NT)).astype(np.float32)).cuda()
+    tab = [lib.WFD_Points_Create((SourcePoint32 * len(p))(*[SourcePoint32(*q) for q in p]), len(p), k) if p else None
+           for k, p in enumerate((spts, rpts))]
+    trc = torch.zeros((nx, NT), device="cuda")
+    torch.cuda.synchronize()
+    vp = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    p = ctypes.c_void_p(g.p)
+    if loop:
+        assert lib.WFD_Prop_Run(p, NT, 1, tab[0], vp(wav), tab[1], vp(trc), NT, 1) == 0
+        assert lib.WFD_Prop_RunLaunches(p) == 1
+    else:
+        s = ctypes.c_void_p(lib.WFD_Prop_Stream(p))
+        for it in range(1, NT + 1):
+            assert lib.WFD_Prop_TimeStepAsync(p, 1, 0) == 0
+            pc = ctypes.c_void_p(ctypes.cast(g.abi.getPCur(g.p), ctypes.c_void_p).value)
+            if tab[0]:
+                assert lib.WFD_Inject(tab[0], pc, vp(wav), it, NT, s) == 0
+            if tab[1]:
+                assert lib.WFD_Extract(tab[1], vp(trc), pc, it, NT, s) == 0
+    assert lib.WFD_Prop_Synchronize(p) == 0
+    keys = ("PCur", "POld", "PSpace") + (() if physics == "Iso" else ("MCur", "MOld", "MSpace"))
+    out = {k: g.arr(k).copy() for k in keys}
+    out["traces"] = trc.cpu().numpy()
+    for t in tab:
+        if t:
+            lib.WFD_Points_Free(t)
+    g.close()
+    return out
+
+
+@pytest.mark.parametrize("physics", ["Iso", "VTI", "TTI"])
+def test_source_points_beyond_the_grid_are_left_out(physics):
+    """As in the loops of the smaller grids, whose tiles hold no such cell."""
+    nx, nz = shape = (1211, 706)
+    inside = [(5 * nz + 9, 1, 1.0)]
+    rec = [(x * nz + 4, x + 1, 1.0) for x in range(nx)]
+    want = _run(physics, shape, True, inside, rec)
+    got = _run(physics, shape, True, inside + [(nx * nz + 1, 1, 3.0), ((nx + 200) * nz + 8, 2, 5.0)], rec)
+    for k in want:
+        assert np.array_equal(got[k], want[k]), k

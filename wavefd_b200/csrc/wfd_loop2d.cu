@@ -277,6 +277,7 @@ __global__ void __launch_bounds__(NT, 2) k_loop2d(Grid g, Fields F, Scratch S, l
     if (threadIdx.x == 0) n_inj = 0;
     __syncthreads();
     for (int gi = threadIdx.x; gi < F.inj.ngroups; gi += NT) {
+        if (F.inj.key[gi] >= g.n) continue;  // outside the grid: in no tile, as in the fused loops
         const int x = (int)(F.inj.key[gi] / g.nz), z = (int)(F.inj.key[gi] % g.nz);
         if ((x / TX * ntz + z / TZ) % (int)gridDim.x == (int)blockIdx.x) inj[atomicAdd(&n_inj, 1)] = gi;
     }
