@@ -290,9 +290,10 @@ const char *WFD_Prop_Message(void *p);
 
 /* Failure-detection hook (no counterpart in the reference): the limit, in ns, of the waits of the TMA
  * step kernels for their tile loads (default 2 s; 0 restores it). A wait that runs out makes the
- * kernel record a timeout in the object's status word, let its copies in flight land and leave; the
- * object then reports WFD_ERR_TIMEOUT. Tests shorten the limit to make a wait run out. Device-wide
- * and synchronous; not for use while other work runs. */
+ * kernel record a timeout in the object's status word (a batched step: the batch's), let its copies in
+ * flight land and leave. The object then reports WFD_ERR_TIMEOUT at its next synchronisation, and no other
+ * object does; after a batched step the batch does, and each object of the batch. Tests shorten the limit to
+ * make a wait run out. Device-wide and synchronous; not for use while other work runs. */
 int WFD_Debug_SetPipelineWait(unsigned long long ns);
 
 /* 1 = bitwise-parity kernels (IEEE order, no FMA), 0 = fast kernels (default) */

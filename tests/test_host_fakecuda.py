@@ -1,0 +1,53 @@
+"""Host side of the library on a stand-in CUDA runtime (fake_cudart.c): failures of single calls, and which kernels
+a call takes. No GPU."""
+import pytest
+
+from tests.fakecuda import run
+
+NAMES = ["Prop3DAcoIsoDenQ_DEO2_FDTD", "Prop2DAcoTTIDenQ_DEO2_FDTD"]
+
+CREATE = r"""
+name, dims = {name!r}, {dims!r}
+free = getattr(lib, name + "_free")
+free.argtypes = [ctypes.c_void_p]
+"""
+
+
+def _create(name):
+    return CREATE.format(name=name, dims=(20, 18 if "3D" in name else 0, 16))
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_every_allocation_of_a_constructor_is_checked(name):
+    """Each allocation in turn fails once: no object, WFD_ERR_ALLOC, nothing left behind; the next object of the
+    process is whole and steps."""
+    n = len(run(_create(name) + "a, p = create(name, *dims)\nfor l in log('alloc'): print(l)\n"))
+    assert n >= 7
+    for k in range(1, n + 1):
+        out = run(_create(name) + r"""
+a, p = create(name, *dims)
+live = fake.fake_live()
+print("NULL" if not p else "OBJECT", lib.WFD_LastError(), lib.WFD_LastErrorMessage().decode(), live)
+a, p = create(name, *dims)
+a.TimeStep(p)
+print("OBJECT" if p else "NULL", lib.WFD_Prop_Status(ctypes.c_void_p(p)))
+""", WAVEFD_B200_FAIL_ALLOC=str(k))
+        assert out[0].startswith("NULL 2 ") and "injected" in out[0] and out[0].endswith(" 0"), (k, out)
+        assert out[1] == "OBJECT 0", (k, out)
+
+
+def test_objects_and_batches_give_their_memory_back():
+    out = run(r"""
+objs = [create("Prop3DAcoIsoDenQ_DEO2_FDTD", 20, 18, 16) for _ in range(2)]
+lib.WFD_Batch_Create.restype = ctypes.c_void_p
+lib.WFD_Batch_Create.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.c_long]
+lib.WFD_Batch_Run.argtypes = [ctypes.c_void_p, ctypes.c_long, ctypes.c_long, ctypes.c_int]
+lib.WFD_Batch_Free.argtypes = [ctypes.c_void_p]
+b = lib.WFD_Batch_Create((ctypes.c_void_p * 2)(*[p for _, p in objs]), 2)
+print(lib.WFD_Batch_Run(b, 3, 1, 1))
+lib.WFD_Batch_Free(b)
+for a, p in objs:
+    a.free(p)
+print(fake.fake_live())
+""")
+    assert out == ["0", "0"]

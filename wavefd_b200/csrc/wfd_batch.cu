@@ -141,6 +141,7 @@ struct Batch {
     int status = WFD_OK;
     std::string message;
     bool tuned = false;
+    std::shared_ptr<StatusWord> word;  // stays set once a wait ran out, as `status` does
     std::vector<float> tune_ms;  // best ms per group and the chosen mode's step
 };
 
@@ -340,14 +341,14 @@ void launch_group(Batch *b, int gi, int k, cudaStream_t s) {
     const int *sel = G.d_sel + k * ns;
     if (G.phys == ISO) {
         if (b->strict) wfd_strict::iso3d_tma_batch(b->gc, (IsoShotDesc *)G.d_desc, sel, G.d_items, G.nitems,
-                                                   b->d_counter + gi, G.grid, s);
+                                                   b->d_counter + gi, G.grid, b->word->w, s);
         else wfd_fast::iso3d_tma_batch(b->gc, (IsoShotDesc *)G.d_desc, sel, G.d_items, G.nitems, b->d_counter + gi,
-                                       G.grid, s);
+                                       G.grid, b->word->w, s);
     } else {
         if (b->strict) wfd_strict::aniso3d_tma_batch(b->gc, G.phys, (AnisoShotDesc *)G.d_desc, sel, G.d_items,
-                                                     G.nitems, b->d_counter + gi, G.grid, s);
+                                                     G.nitems, b->d_counter + gi, G.grid, b->word->w, s);
         else wfd_fast::aniso3d_tma_batch(b->gc, G.phys, (AnisoShotDesc *)G.d_desc, sel, G.d_items, G.nitems,
-                                         b->d_counter + gi, G.grid, s);
+                                         b->d_counter + gi, G.grid, b->word->w, s);
     }
 }
 
@@ -428,7 +429,7 @@ void order_props_after(Batch *b) {
 
 int batch_sync(Batch *b) {
     if (int rc = bcheck(b, cudaStreamSynchronize(b->stream), "batch synchronize")) return rc;
-    if (wfd::take_status())
+    if (b->word->set())
         return bfail(b, WFD_ERR_TIMEOUT, "a batched step kernel timed out waiting for its tile loads");
     return WFD_OK;
 }
@@ -458,6 +459,8 @@ int batch_run(Batch *b, long nsteps, long it0, bool graph) {
         swap_all(b);
     }
     if (int rc = bcheck(b, cudaGetLastError(), "batch step launch")) return rc;
+    for (Prop *p : b->props)
+        if (p->batch_words.empty() || p->batch_words.back() != b->word) p->batch_words.push_back(b->word);
     order_props_after(b);
     return WFD_OK;
 }
@@ -665,7 +668,8 @@ Batch *batch_create(Prop *const *props, long n) {
         b->groups[p->phys].shots.push_back((int)i);
     }
     b->acq.resize(n);
-    bool ok = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) == cudaSuccess;
+    b->word = make_status_word();
+    bool ok = b->word && cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) == cudaSuccess;
     for (int i = 0; i < 3 && ok; i++)
         ok = cudaStreamCreateWithFlags(&b->side[i], cudaStreamNonBlocking) == cudaSuccess &&
              cudaEventCreateWithFlags(&b->ev_join[i], cudaEventDisableTiming) == cudaSuccess;

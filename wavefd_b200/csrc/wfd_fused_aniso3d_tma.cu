@@ -724,13 +724,13 @@ bool aniso3d_tma_describe(const Grid &g, int phys, const Fields &F, int xchunk, 
 }
 
 void aniso3d_tma_batch(const Grid &gc, int phys, const AnisoShotDesc *shots, const int *sel, const int2 *items,
-                       int nitems, int *counter, int grid, cudaStream_t s) {
+                       int nitems, int *counter, int grid, unsigned *status, cudaStream_t s) {
     if (phys == TTI) {
         aniso_grid_cap<TTI, false>();
-        k_aniso3d_tma<TTI, false, true><<<grid, NT, SMEM_BYTES, s>>>(gc, batch_fields(), AnisoMaps{}, 0, 0, 0, 1, shots,
+        k_aniso3d_tma<TTI, false, true><<<grid, NT, SMEM_BYTES, s>>>(gc, batch_fields(status), AnisoMaps{}, 0, 0, 0, 1, shots,
                                                                      sel, items, nitems, counter);
     } else {
-        vti3d_tma_batch(gc, shots, sel, items, nitems, counter, grid, s);
+        vti3d_tma_batch(gc, shots, sel, items, nitems, counter, grid, status, s);
     }
 }
 

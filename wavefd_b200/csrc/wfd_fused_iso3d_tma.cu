@@ -692,9 +692,9 @@ bool iso3d_tma_describe(const Grid &g, const Fields &F, int xchunk, IsoShotDesc 
 }
 
 void iso3d_tma_batch(const Grid &gc, const IsoShotDesc *shots, const int *sel, const int2 *items, int nitems,
-                     int *counter, int grid, cudaStream_t s) {
-    k_iso3d_tma<true><<<grid, NT, SMEM_BYTES, s>>>(gc, batch_fields(), IsoMaps{}, 0, 0, 0, 1, shots, sel, items, nitems,
-                                                   counter);
+                     int *counter, int grid, unsigned *status, cudaStream_t s) {
+    k_iso3d_tma<true><<<grid, NT, SMEM_BYTES, s>>>(gc, batch_fields(status), IsoMaps{}, 0, 0, 0, 1, shots, sel, items,
+                                                   nitems, counter);
 }
 
 void iso3d_set_pipeline_wait(unsigned long long ns) {

@@ -612,10 +612,10 @@ bool vti3d_tma_describe(const Grid &g, const Fields &F, int xchunk, AnisoShotDes
 }
 
 void vti3d_tma_batch(const Grid &gc, const AnisoShotDesc *shots, const int *sel, const int2 *items, int nitems,
-                     int *counter, int grid, cudaStream_t s) {
+                     int *counter, int grid, unsigned *status, cudaStream_t s) {
     vti_grid_cap<false>();
-    k_vti3d_tma<false, true><<<grid, NT, SMEM_BYTES, s>>>(gc, batch_fields(), AnisoMaps{}, 0, 0, 0, 1, shots, sel, items,
-                                                         nitems, counter);
+    k_vti3d_tma<false, true><<<grid, NT, SMEM_BYTES, s>>>(gc, batch_fields(status), AnisoMaps{}, 0, 0, 0, 1, shots, sel,
+                                                         items, nitems, counter);
 }
 
 void vti3d_set_pipeline_wait(unsigned long long ns) {

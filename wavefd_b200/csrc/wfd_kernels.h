@@ -54,20 +54,14 @@ struct Fields {
     float *v, *b, *q, *eps, *eta, *f, *st, *ct, *sp, *cp;
     float *pcur, *pold, *pspace, *mcur, *mold, *mspace;
     float *illum;  // source illumination sum (sum over steps of pCur^2), or nullptr
-    unsigned *status;  // set to 1 by a kernel whose bounded wait ran out (status_word())
+    unsigned *status;  // set to 1 by a kernel whose bounded wait ran out (a StatusWord)
     StepInject inj;
     StepEpilogue epi;
 };
 
-// The process-wide status word of the step kernels' bounded waits: mapped pinned memory, so that reading it
-// after a stream synchronisation costs no copy (six copies of per-kernel device words took 60 of the 79 us
-// of a synchronisation). nullptr when it cannot be allocated.
-unsigned *status_word();
-bool take_status();  // whether a wait ran out since the last call
-
-inline Fields batch_fields() {  // batched launches: the arrays come from the shots' descriptors
+inline Fields batch_fields(unsigned *status) {  // batched launches: the arrays come from the shots' descriptors
     Fields F{};
-    F.status = status_word();
+    F.status = status;
     return F;
 }
 
@@ -156,17 +150,19 @@ struct TileInfo {
     bool vti3d_tma_describe(const wfd::Grid &g, const wfd::Fields &F, int xchunk, wfd::AnisoShotDesc *d, \
                             wfd::TileInfo *t);                                                           \
     void vti3d_tma_batch(const wfd::Grid &gc, const wfd::AnisoShotDesc *shots, const int *sel,          \
-                         const int2 *items, int nitems, int *counter, int grid, cudaStream_t s);        \
+                         const int2 *items, int nitems, int *counter, int grid, unsigned *status,       \
+                         cudaStream_t s);                                                               \
     /* batched launches over many shots (descriptors and items in device memory) */                     \
     bool iso3d_tma_describe(const wfd::Grid &g, const wfd::Fields &F, int xchunk, wfd::IsoShotDesc *d,   \
                             wfd::TileInfo *t);                                                           \
     void iso3d_tma_batch(const wfd::Grid &gc, const wfd::IsoShotDesc *shots, const int *sel,            \
-                         const int2 *items, int nitems, int *counter, int grid, cudaStream_t s);        \
+                         const int2 *items, int nitems, int *counter, int grid, unsigned *status,       \
+                         cudaStream_t s);                                                               \
     bool aniso3d_tma_describe(const wfd::Grid &g, int phys, const wfd::Fields &F, int xchunk,           \
                               wfd::AnisoShotDesc *d, wfd::TileInfo *t);                                  \
     void aniso3d_tma_batch(const wfd::Grid &gc, int phys, const wfd::AnisoShotDesc *shots,              \
                            const int *sel, const int2 *items, int nitems, int *counter, int grid,       \
-                           cudaStream_t s);                                                              \
+                           unsigned *status, cudaStream_t s);                                                              \
     void iso3d_set_pipeline_wait(unsigned long long ns);                                                 \
     void vti3d_set_pipeline_wait(unsigned long long ns);                                                 \
     void aniso3d_set_pipeline_wait(unsigned long long ns);                                               \

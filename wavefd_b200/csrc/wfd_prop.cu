@@ -77,22 +77,15 @@ int prop_fail(Prop *p, int code, const std::string &msg) {
     return code;
 }
 
-unsigned *status_word() {
-    static unsigned *const word = [] {
-        void *p = nullptr;
-        if (cudaHostAlloc(&p, sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
-            cudaGetLastError();
-            return (unsigned *)nullptr;
-        }
-        *(unsigned *)p = 0;
-        return (unsigned *)p;  // kept until the process ends: kernels of any object may write it
-    }();
-    return word;
-}
-
-bool take_status() {
-    unsigned *w = status_word();
-    return w && __atomic_exchange_n(w, 0u, __ATOMIC_ACQ_REL) != 0;
+std::shared_ptr<StatusWord> make_status_word() {
+    auto s = std::make_shared<StatusWord>();
+    if (wfd::dMallocHost(&s->w, sizeof(unsigned)) != cudaSuccess) {
+        cudaGetLastError();
+        s->w = nullptr;
+        return nullptr;
+    }
+    *s->w = 0;
+    return s;
 }
 
 static int check_cuda(Prop *p, cudaError_t e, const char *what) {
@@ -144,7 +137,7 @@ Fields Prop::fields() const {
     F.mold = field[F_MOLD];
     F.mspace = field[F_MSPACE];
     F.illum = illum;
-    F.status = status_word();
+    F.status = word->w;
     F.inj = inj;
     F.epi = epi;
     return F;
@@ -214,13 +207,18 @@ Prop *prop_create(int ndim, int phys, long fs, long nthread, long nx, long ny, l
             return nullptr;
         }
     }
+    p->word = make_status_word();
+    if (!p->word) {
+        set_global_error(WFD_ERR_ALLOC, std::string("status word allocation failed") + alloc_injected_note());
+        prop_destroy(p);
+        return nullptr;
+    }
     if (cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking) != cudaSuccess) {
         set_global_error(WFD_ERR_CUDA, "stream creation failed");
         prop_destroy(p);
         return nullptr;
     }
     p->own_stream = true;
-    status_word();  // allocated here, not by a step that may be under capture
     for (int f = 0; f < F_COUNT; f++) {
         if (!p->alloc[f]) continue;
 #if CUDART_VERSION >= 13000
@@ -330,8 +328,11 @@ void prop_setup_q(Prop *p, float freqQ, float qMin, float qInterior) {
 // ---------------------------------------------------------------------------------------------
 int prop_sync(Prop *p) {
     if (int rc = check_cuda(p, cudaStreamSynchronize(p->stream), "synchronize")) return rc;
-    // the TMA kernels' status word: a bounded wait that ran out
-    if (take_status())
+    // a bounded wait of the step kernels that ran out: in the object's own steps or a batch's
+    bool timeout = p->word->take();
+    for (const auto &w : p->batch_words) timeout = timeout || w->set();
+    p->batch_words.clear();
+    if (timeout)
         return prop_fail(p, WFD_ERR_TIMEOUT, "a fused step kernel timed out waiting for its tile loads");
     return WFD_OK;
 }
@@ -339,7 +340,6 @@ int prop_sync(Prop *p) {
 int prop_step(Prop *p, bool linear, bool sync) {
     Grid g = p->grid();
     Fields F = p->fields();
-    if (!F.status) return prop_fail(p, WFD_ERR_ALLOC, "status word allocation failed");
     // the step kernels read the epilogue's arrays 16 (Iso) or 8 bytes at a time: arrays at other
     // alignments take the separate kernels after the step
     auto a16 = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };

@@ -3,7 +3,9 @@
 
 #include <cuda_runtime.h>
 
+#include <memory>
 #include <string>
+#include <vector>
 
 #include "wavefd_b200.h"
 #include "wfd_kernels.h"
@@ -17,6 +19,19 @@ enum FieldId {
 };
 
 // Status codes (WFD_OK, WFD_ERR_*) are the add-on API's, from the public header.
+
+// The word that step kernels set when a bounded wait ran out: an object's own steps its own, a batch's launches the
+// batch's. Mapped pinned memory, so that reading it after a stream synchronisation costs no copy (six
+// copies of per-kernel device words took 60 of the 79 us of a synchronisation).
+struct StatusWord {
+    unsigned *w = nullptr;
+    ~StatusWord() {
+        if (w) cudaFreeHost(w);
+    }
+    bool set() const { return __atomic_load_n(w, __ATOMIC_ACQUIRE) != 0; }
+    bool take() { return __atomic_exchange_n(w, 0u, __ATOMIC_ACQ_REL) != 0; }
+};
+std::shared_ptr<StatusWord> make_status_word();  // empty when it cannot be allocated
 
 struct Prop {
     int ndim = 3;
@@ -45,6 +60,9 @@ struct Prop {
     StepInject inj{};      // a source injection for the step kernel to apply (WFD_Prop_Run), or none
     StepEpilogue epi{};    // Born injection / imaging condition to apply right after the next step, or none
     bool inject_done = false;  // the last step kernel applied `inj`
+    std::shared_ptr<StatusWord> word;  // of this object's own steps
+    // of the batches that stepped this object since its last synchronisation
+    std::vector<std::shared_ptr<StatusWord>> batch_words;
 
     long ncells() const { return nx * ny * nz; }
     size_t alloc_bytes() const;  // of one field's allocation
