@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(NT, 3)
 
     const long total = (long)ntz0 * nty0 * nch0;
     unsigned gseq = 0;                  // groups consumed so far by this CTA
-    unsigned out_from = 0, out_to = 0;  // groups issued but not yet consumed (thread 0)
+    unsigned out_from = 0, out_to = 0;  // groups issued but not yet consumed (by whoever issues them)
     const int zq = lane & 7;
     const int row = 4 * warp + (lane >> 3);
 
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(NT, 3)
                 *(volatile unsigned *)F.status = 1u;
             }
             // a group whose wait ran out may still be in flight: the drain below waits for it
-            if (tid == 0 && landed) out_from = gs + 1;
+            if ((RAG || tid == 0) && landed) out_from = gs + 1;
             float *st = sm + slot * STAGE;
             slot = slot + 1 == NS ? 0u : slot + 1;
             par ^= slot == 0 ? 1u : 0u;
@@ -598,10 +598,10 @@ __global__ void __launch_bounds__(NT, 3)
         gseq += ngroups;
         if (stop) break;
     }
-    if (RAG) {
-        cp_async_drain();
-    } else if (*abort_flag && tid == 0) {
-        // let copies still in flight land before the CTA leaves (bounded)
+    if (RAG) cp_async_drain();
+    if (*abort_flag && (RAG || tid == 0)) {
+        // let copies still in flight land before the CTA leaves, and the arrivals on the barriers that follow
+        // a thread's cp.async (bounded)
         for (unsigned gs = out_from; gs < out_to; gs++) mbar_wait(&bars[gs % NS], (gs / NS) & 1u, 100000000ull);
     }
 }
