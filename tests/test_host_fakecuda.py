@@ -51,3 +51,25 @@ for a, p in objs:
 print(fake.fake_live())
 """)
     assert out == ["0", "0"]
+
+
+@pytest.mark.parametrize("strict", ["0", "1"])
+@pytest.mark.parametrize("name,dims", [("Prop3DAcoIsoDenQ_DEO2_FDTD", (24, 20, 17)),
+                                       ("Prop3DAcoIsoDenQ_DEO2_FDTD", (24, 20, 16)),
+                                       ("Prop3DAcoVTIDenQ_DEO2_FDTD", (24, 20, 16)),
+                                       ("Prop3DAcoTTIDenQ_DEO2_FDTD", (24, 20, 16)),
+                                       ("Prop2DAcoVTIDenQ_DEO2_FDTD", (24, 0, 16)),
+                                       ("Prop2DAcoTTIDenQ_DEO2_FDTD", (24, 0, 16))])
+def test_a_second_device_steps_too(name, dims, strict):
+    """Kernels with more than 48 KB of shared memory need it granted on each device that runs them."""
+    out = run(f"""
+for dev in (0, 1, 0):
+    fake.cudaSetDevice(dev)
+    a, p = create({name!r}, *{dims!r})
+    fake.fake_reset()
+    a.TimeStep(p)
+    print(lib.WFD_Prop_Status(ctypes.c_void_p(p)), lib.WFD_Prop_Run(p, 3, 1, None, None, None, None, 3, 0))
+    print(*launches())
+""", WAVEFD_B200_STRICT=strict)
+    assert out[::2] == ["0 0"] * 3, out
+    assert out[1] == out[3] == out[5] != ""

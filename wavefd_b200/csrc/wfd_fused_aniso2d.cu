@@ -294,7 +294,8 @@ __global__ void __launch_bounds__(NT) k_aniso2d_run(Grid g, Fields F, long nstep
 
 template <int PHYS, bool LINEAR>
 bool launch2(const Grid &g, const Fields &F, cudaStream_t s) {
-    static bool attr = false;
+    static PerDevice<bool> attrs;
+    bool &attr = attrs.here();
     if (!attr) {
         if (cudaFuncSetAttribute(k_aniso2d_fused<PHYS, LINEAR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)SMEM_BYTES) != cudaSuccess)
@@ -312,11 +313,12 @@ bool launch2(const Grid &g, const Fields &F, cudaStream_t s) {
 int aniso2d_run(const Grid &g, int phys, const Fields &F, long nsteps, long it0, const RunExtract &ex,
                 unsigned *sync_words, cudaStream_t s) {
     if (g.ndim != 2 || (phys != VTI && phys != TTI)) return -1;
-    // co-resident CTAs (0: no cooperative launch, or the shared memory cannot be granted)
-    static int cap[2] = {-1, -1};
+    // co-resident CTAs, plus one (1: no cooperative launch, or the shared memory cannot be granted; 0: not asked yet)
+    static PerDevice<int> caps[2];
     const int which = phys == TTI ? 1 : 0;
     const void *fn = which ? (const void *)k_aniso2d_run<TTI> : (const void *)k_aniso2d_run<VTI>;
-    if (cap[which] < 0) {
+    int &cap1 = caps[which].here();
+    if (!cap1) {
         int dev = 0, sms = 0, per = 0, coop = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
@@ -324,14 +326,15 @@ int aniso2d_run(const Grid &g, int phys, const Fields &F, long nsteps, long it0,
         if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES) == cudaSuccess)
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, NT, SMEM_BYTES);
         cudaGetLastError();
-        cap[which] = coop ? sms * per : 0;
+        cap1 = 1 + (coop ? sms * per : 0);
     }
-    if (cap[which] <= 0) return -1;
+    const int cap = cap1 - 1;
+    if (cap <= 0) return -1;
     const long ntiles = ((g.nz + TZ - 1) / TZ) * ((g.nx + TX - 1) / TX);
 #if !WFD_STRICT
-    if (ntiles > cap[which]) return -1;  // wfd_loop2d.cu takes those
+    if (ntiles > cap) return -1;  // wfd_loop2d.cu takes those
 #endif
-    const int grid = (int)(ntiles < cap[which] ? ntiles : cap[which]);
+    const int grid = (int)(ntiles < cap ? ntiles : cap);
     Grid gg = g;
     Fields FF = F;
     long ns = nsteps, i0 = it0;

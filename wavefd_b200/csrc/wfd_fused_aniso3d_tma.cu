@@ -642,7 +642,8 @@ bool aniso_maps(const Grid &g, int phys, const Fields &F, CUtensorMap *m) {
 
 template <int PHYS, bool LINEAR>
 int aniso_grid_cap() {
-    static int cap = 0;
+    static PerDevice<int> caps;
+    int &cap = caps.here();
     if (!cap) {
         for (auto kern : {k_aniso3d_tma<PHYS, LINEAR, false>, k_aniso3d_tma<PHYS, LINEAR, true>,
                           k_aniso3d_tma<PHYS, LINEAR, false, true>})

@@ -469,8 +469,13 @@ int iso2d_run(const Grid &g, const Fields &F, long nsteps, long it0, const RunEx
               cudaStream_t s) {
     if (g.ndim != 2) return -1;
     // co-resident CTAs of the two forms (0: no cooperative launch, or the form is not in this build)
-    static int cap = -1, cap_res = 0;
-    if (cap < 0) {
+    struct Cap {
+        bool known;
+        int run, res;
+    };
+    static PerDevice<Cap> caps;
+    Cap &c = caps.here();
+    if (!c.known) {
         int dev = 0, sms = 0, per = 0, per_res = 0, coop = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
@@ -479,9 +484,9 @@ int iso2d_run(const Grid &g, const Fields &F, long nsteps, long it0, const RunEx
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_iso2d_run, NT, 0);
 #endif
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_res, k_iso2d_run_res, NT, 0);
-        cap = coop ? sms * per : 0;
-        cap_res = coop ? sms * per_res : 0;
+        c = Cap{true, coop ? sms * per : 0, coop ? sms * per_res : 0};
     }
+    const int cap = c.run, cap_res = c.res;
     const long ntiles = ((g.nz + TZ - 1) / TZ) * ((g.nx + TX - 1) / TX);
     const bool resident = ntiles <= cap_res && F.inj.ngroups <= MAX_INJ;
     if (!resident && cap <= 0) return -1;

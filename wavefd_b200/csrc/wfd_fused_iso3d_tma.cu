@@ -611,7 +611,8 @@ __global__ void __launch_bounds__(NT, 3)
 namespace {
 
 int iso_grid_cap() {
-    static int cap = 0;
+    static PerDevice<int> caps;
+    int &cap = caps.here();
     if (!cap) {
         int dev = 0, sms = 0, per = 0;
         for (auto kern : {k_iso3d_tma<false>, k_iso3d_tma<true>, k_iso3d_tma<false, true>, k_iso3d_tma<false, false, true>})

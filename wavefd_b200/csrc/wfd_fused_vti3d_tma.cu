@@ -534,7 +534,8 @@ bool vti_maps(const Grid &g, const Fields &F, CUtensorMap *m) {
 
 template <bool LINEAR>
 int vti_grid_cap() {
-    static int cap = 0;
+    static PerDevice<int> caps;
+    int &cap = caps.here();
     if (!cap) {
         for (auto kern : {k_vti3d_tma<LINEAR, false>, k_vti3d_tma<LINEAR, true>, k_vti3d_tma<LINEAR, false, true>})
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);

@@ -93,6 +93,18 @@ struct alignas(64) AnisoShotDesc {
     int nx, ny, nz, ntz, nty, xchunk;
 };
 
+// What a launcher finds out once for a device and keeps (a kernel's shared-memory grant holds for the device it was
+// made on): the current device's value.
+template <class T>
+struct PerDevice {
+    T v[64] = {};
+    T &here() {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        return v[dev & 63];
+    }
+};
+
 // Tile geometry and capacity of a TMA step kernel, for the batch planner.
 struct TileInfo {
     int tz, ty;      // (z, y) cross-section of a tile
