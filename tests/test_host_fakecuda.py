@@ -73,3 +73,36 @@ for dev in (0, 1, 0):
 """, WAVEFD_B200_STRICT=strict)
     assert out[::2] == ["0 0"] * 3, out
     assert out[1] == out[3] == out[5] != ""
+
+
+def _two_pass(physics, sizes):
+    """The kernels of a step, for (nx, ny, nz) with nz % 4 != 0."""
+    return run(f"""
+for size in {sizes!r}:
+    a, p = create("Prop3DAco{physics}DenQ_DEO2_FDTD", *size)
+    fake.fake_reset()
+    a.TimeStep(p)
+    print(*launches())
+    a.free(p)
+""")
+
+
+@pytest.mark.parametrize("physics", ["VTI", "TTI"])
+def test_two_pass_kernels_by_size(physics):
+    """Marching kernels for a million cells and more in well filled tiles, one thread a cell elsewhere (thin grids
+    took up to 3.9 times as long on the marching kernels)."""
+    from tests.test_gpu_pass3d import SHAPES
+    marching = [(nx, ny, nz) for nz, ny, nx in SHAPES] + [(203, 181, 251), (250, 90, 90), (16, 400, 301), (80, 112, 126)]
+    cells = [(12000, 9, 10), (3000, 17, 33), (2000, 33, 17), (20, 20, 3001), (40, 33, 1001), (300, 18, 301), (300, 300, 33),
+             (600, 33, 65), (9, 1000, 301), (101, 100, 101), (64, 60, 67)]
+    for line in _two_pass(physics, marching):
+        assert "k_pass1_3d" in line and "k_pass2_3d" in line, line
+    for size, line in zip(cells, _two_pass(physics, cells)):
+        assert "k_pass1I" in line and "k_pass2I" in line and "_3d" not in line, (size, line)
+
+
+def test_two_pass_kernels_between_the_lines():
+    """Where only one physics gains."""
+    sizes = [(400, 180, 50), (300, 300, 50), (150, 113, 135)]
+    assert all("_3d" not in line for line in _two_pass("VTI", sizes))
+    assert all("k_pass1_3d" in line for line in _two_pass("TTI", sizes))

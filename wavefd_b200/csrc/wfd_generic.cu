@@ -596,7 +596,7 @@ MPtr3 m3(float *const *a) { return MPtr3{{a[0], a[1], a[2]}}; }
 
 // ---------------------------------------------------------------------------------------------
 void pass1(const Grid &g, int phys, const Fields &F, const Scratch &S, cudaStream_t s) {
-    if (pass3d_takes(g)) return pass1_3d(g, phys, F, S, s);
+    if (pass3d_takes(g, phys)) return pass1_3d(g, phys, F, S, s);
     const unsigned nb = blocks_for(g.n);
     if (phys == ISO) k_pass1<ISO><<<nb, kThreads, 0, s>>>(g, F, S);
     else if (phys == VTI) k_pass1<VTI><<<nb, kThreads, 0, s>>>(g, F, S);
@@ -604,7 +604,7 @@ void pass1(const Grid &g, int phys, const Fields &F, const Scratch &S, cudaStrea
 }
 
 void pass2(const Grid &g, int phys, int linear, const Fields &F, const Scratch &S, cudaStream_t s) {
-    if (pass3d_takes(g)) return pass2_3d(g, phys, linear, F, S, s);
+    if (pass3d_takes(g, phys)) return pass2_3d(g, phys, linear, F, S, s);
     const unsigned nb = blocks_for(g.n);
     if (phys == ISO) k_pass2<ISO, false><<<nb, kThreads, 0, s>>>(g, F, S);
     else if (phys == VTI && linear) k_pass2<VTI, true><<<nb, kThreads, 0, s>>>(g, F, S);

@@ -120,8 +120,8 @@ struct TileInfo {
     void pass1(const wfd::Grid &g, int phys, const wfd::Fields &F, const wfd::Scratch &S, cudaStream_t s); \
     void pass2(const wfd::Grid &g, int phys, int linear, const wfd::Fields &F, const wfd::Scratch &S,    \
                cudaStream_t s);                                                                          \
-    /* the same two passes for the larger 3D grids (pass3d_takes) */                                     \
-    bool pass3d_takes(const wfd::Grid &g);                                                               \
+    /* the same two passes for larger 3D grids (pass3d_takes) */                                         \
+    bool pass3d_takes(const wfd::Grid &g, int phys);                                                     \
     void pass1_3d(const wfd::Grid &g, int phys, const wfd::Fields &F, const wfd::Scratch &S, cudaStream_t s); \
     void pass2_3d(const wfd::Grid &g, int phys, int linear, const wfd::Fields &F, const wfd::Scratch &S, \
                   cudaStream_t s);                                                                       \

@@ -361,11 +361,23 @@ int chunk_of(const Grid &g, dim3 &grid) {
 
 }  // namespace
 
-// Grids of a million cells and more. Smaller ones stay in L2 and are bound by the latency of a launch, which
-// one thread a cell (wfd_generic.cu) hides better: TTI 80 x 75 x 69 21.2 us a step against 23.0 here,
-// 100 x 110 x 90 41.6 against 36.9.
-bool pass3d_takes(const Grid &g) {
-    return g.ndim == 3 && g.n >= 1000000 && (g.ny + TY - 1) / TY <= 65535 && (g.nz + TZ - 1) / TZ < 2147483647L;
+// Grids of a million cells and more whose tiles are well filled; the others take one thread a cell
+// (wfd_generic.cu). Smaller grids stay in L2 and are bound by the latency of a launch, which one thread a cell hides
+// better: TTI 80 x 75 x 69 21.2 us a step there and 23.0 here (100 x 110 x 90 41.6 and 36.9: the times cross below
+// the line, but between few cells and many the filling of the tiles moves the crossing more than the count).
+// A tile costs the same however much of it is computed, so the second rule is on a plane's tile cells per computed
+// cell, r. us a step there and here, on both sides of each line: VTI (r <= 1.32) 250 x 90 x 90 r 1.31 78.9, 74.7;
+// 160 x 140 x 101 r 1.44 88.6, 88.2; 300 x 300 x 50 r 1.45 172, 182; 12000 x 9 x 10 r 85 33.9, 131.5. TTI (1.6)
+// 400 x 180 x 50 r 1.55 172.8, 162.9; 101 x 100 x 101 r 1.61 46.0, 47.4; 300 x 70 x 70 r 1.88 67.7, 72.4; Iso (1.5)
+// 150 x 113 x 136 r 1.48 50.4, 45.9; 300 x 300 x 44 r 1.67 90.8, 99.6. Below 12 planes the zeros that each CTA
+// writes on the planes beside the computed ones show: VTI 9 x 1000 x 301 36.5, 41.3; 14 x 310 x 319 32.4, 31.7.
+bool pass3d_takes(const Grid &g, int phys) {
+    if (g.ndim != 3 || g.n < 1000000 || g.nx < 12) return false;
+    const long nty = (g.ny + TY - 1) / TY, ntz = (g.nz + TZ - 1) / TZ;
+    if (nty > 65535 || ntz >= 2147483647L) return false;
+    const double staged = (double)(ntz * TZ) * (double)(nty * TY);
+    const double computed = (double)(g.ny - 8) * (double)(g.nz - (g.fs ? 4 : 8));
+    return staged <= (phys == TTI ? 1.6 : (phys == VTI ? 1.32 : 1.5)) * computed;
 }
 
 void pass1_3d(const Grid &g, int phys, const Fields &F, const Scratch &S, cudaStream_t s) {
