@@ -106,3 +106,24 @@ def test_two_pass_kernels_between_the_lines():
     sizes = [(400, 180, 50), (300, 300, 50), (150, 113, 135)]
     assert all("_3d" not in line for line in _two_pass("VTI", sizes))
     assert all("k_pass1_3d" in line for line in _two_pass("TTI", sizes))
+
+
+@pytest.mark.parametrize("call", ["injectdata", "extractdata"])
+def test_host_points_copied_where_one_thread_reads_many(call):
+    """Drop-in calls with host arrays: (groups, points a group) and whether the values go to the device by a copy."""
+    want = {(1, 1): 0, (1, 64): 0, (1, 65): 1, (2, 512): 1, (40, 64): 0, (4096, 1): 0, (4097, 1): 1, (1, 5000): 1}
+    out = run(f"""
+import numpy as np
+from wavefd_b200 import spacetime
+for groups, per in {list(want)!r}:
+    pts = np.zeros(groups * per, spacetime.SOURCEPOINT32)
+    one, many = ("iu", "ir") if {call!r} == "injectdata" else ("ir", "iu")
+    pts[one], pts[many], pts["c"] = np.repeat(np.arange(1, groups + 1), per), np.arange(groups * per) % 4000 + 1, 1.0
+    field, data = np.zeros(8000, np.float32), np.zeros((8000, 2), np.float32)
+    for again in range(2):  # the first call also uploads the points
+        fake.fake_reset()
+        if {call!r} == "injectdata": spacetime.injectdata(field, [pts], data, 1)
+        else: spacetime.extractdata(data, field, 1, [pts])
+    print(len(log("copy")), len(launches()))
+""")
+    assert out == [f"{n} 1" for n in want.values()], out

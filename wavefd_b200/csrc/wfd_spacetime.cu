@@ -156,6 +156,7 @@ struct CachedTable {
     int by_receiver = 0;
     std::vector<PointsT<T>> raw;       // the caller's points, partition by partition
     std::vector<long> counts;          // points per partition
+    long longest = 0;                  // points of the largest group
     unsigned long long last_use = 0;
     T *d_src = nullptr;                    // device staging (points)
     T *h_dst = nullptr, *h_src = nullptr;  // pinned host staging (groups, points), mapped
@@ -164,7 +165,11 @@ struct CachedTable {
 // Host loops over the points of a drop-in call use up to the caller's thread count (the reference's
 // nthreads argument) once they are long enough to pay for it.
 constexpr long kParallelPoints = 8192;
-constexpr long kMappedPoints = 4096;
+// Values that the kernel reads from mapped pinned memory itself: up to kMappedPoints of them, and up to kMappedRun by one
+// thread, which reads a group's one after another at 0.14 us each over the bus (0.03 from device memory, after a
+// copy of 5 to 10 us). Extraction with host arrays, groups x points, us a call read so and copied: 1 x 32 34.5,
+// 35.1; 1 x 64 39.4, 36.1; 64 x 64 57.7, 61.9; 1 x 128 48.1, 36.4; 8 x 512 120, 72; 1 x 4096 601, 153.
+constexpr long kMappedPoints = 4096, kMappedRun = 64;
 
 template <class T>
 bool same_points(const CachedTable<T> &e, int by_receiver, void **partitions, size_t npartitions,
@@ -223,6 +228,7 @@ CachedTable<T> *lookup(TableCache<T> &cache, int by_receiver, void **partitions,
     e->raw = flatten<T>(partitions, npartitions, npoints);
     e->counts.assign(npoints, npoints + npartitions);
     build(e->t, e->raw, by_receiver);
+    for (long g = 0; g < e->t.ngroups; g++) e->longest = std::max(e->longest, e->t.start[g + 1] - e->t.start[g]);
     const size_t ng = (size_t)e->t.ngroups, np = (size_t)e->t.npoints;
     bool ok = upload(e->t, s);
     ok = ok && wfd::dMallocAsync(&e->d_src, sizeof(T) * (np + 1), s) == cudaSuccess;
@@ -268,10 +274,9 @@ void dropin(int by_receiver, T *dst, long dst_stride, long dst_off, const T *src
     const bool dst_dev = device_accessible(dst);
     const bool src_dev = device_accessible(src);
     const long ng = t.ngroups, np = t.npoints;
-    // The kernel reads and writes the pinned staging itself: each written location once and coalesced, and
-    // up to kMappedPoints values read by one thread per group. More go through the device (a copy's
-    // fixed cost, about 10 us with its wait, is then less than the scattered reads).
-    const bool copy = np > kMappedPoints;
+    // The kernel reads and writes the pinned staging itself: each written location once and coalesced, and the
+    // values read where they are few. More go through the device.
+    const bool copy = np > kMappedPoints || e->longest > kMappedRun;
     if (!src_dev) {
 #pragma omp parallel for num_threads(nth) if (np >= kParallelPoints) schedule(static)
         for (long j = 0; j < np; j++) e->h_src[j] = src[t.other[j] * src_stride + src_off];
