@@ -263,7 +263,7 @@ struct Sep {
 };
 
 template <int K>
-__global__ void __launch_bounds__(Sep<K>::NT, Sep<K>::NT > 512 ? 1 : (Sep<K>::NT > 256 ? 1 : 3))
+__global__ void __launch_bounds__(Sep<K>::NT, Sep<K>::NT > 256 ? 1 : 3)
     k_wavefieldsep(long ncols, int nz, int isfwi, const float *__restrict__ v_, const float *__restrict__ b_,
                    const float *__restrict__ pold, const float *__restrict__ mold, const float *__restrict__ dp,
                    const float *__restrict__ dm, float *__restrict__ dv) {
@@ -274,7 +274,8 @@ __global__ void __launch_bounds__(Sep<K>::NT, Sep<K>::NT > 512 ? 1 : (Sep<K>::NT
     float2 *bu = sm + (2 * slot) * C::BUF, *bv = bu + C::BUF;
     float2 *G = sm + C::O_G, *W = sm + C::O_W, *dc = sm + C::O_DC + 2 * slot;
 
-    // twiddles, then the operator's taps through the same transform
+    // Twiddles, then the operator's taps through the same transform. The taps are formed by all threads together (a
+    // cotangent in double is long, and a CTA of several columns would form each one several times).
     if (!C::BIG) {
         for (int i = threadIdx.x; i < L; i += C::NT) {
             int m = L, o = i;  // stage length and offset inside the stage
@@ -289,15 +290,17 @@ __global__ void __launch_bounds__(Sep<K>::NT, Sep<K>::NT > 512 ? 1 : (Sep<K>::NT
                 W[i] = make_float2((float)c, (float)s);
             }
         }
-        __syncthreads();
     }
     {
+        float *taps = reinterpret_cast<float *>(G);
+        for (int i = threadIdx.x; i < L; i += C::NT) taps[i] = C::tap(2 * (i < L / 2 ? i : i - L) + 1, nz);
+        __syncthreads();
         float2 u[8], v[8];
 #pragma unroll
-        for (int r = 0; r < 8; r++) {
-            const int i = t + r * T, k = i < L / 2 ? i : i - L;
-            v[r] = make_float2(C::tap(2 * k + 1, nz), 0.0f);
-            u[r] = make_float2(C::tap(2 * k - 1, nz), 0.0f);
+        for (int r = 0; r < 8; r++) {  // v: distance 2i + 1 (i from -L/2 to L/2 - 1), u: 2i - 1
+            const int i = t + r * T;
+            v[r] = make_float2(taps[i], 0.0f);
+            u[r] = make_float2(i == L / 2 ? 0.0f : taps[(i + L - 1) % L], 0.0f);
         }
         C::template forward<0, false>(u, v, bu, bv, W, t);
         if (slot == 0) {
@@ -402,14 +405,19 @@ template <int K>
 bool launch(const Grid &g, long isfwi, const Fields &F, const float *dp, const float *dm, float *dv, cudaStream_t s) {
     using C = Sep<K>;
     const long ncols = g.nx * g.ny;
-    if (cudaFuncSetAttribute(k_wavefieldsep<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM) != cudaSuccess)
-        return false;
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_wavefieldsep<K>, C::NT, C::SMEM) != cudaSuccess || per < 1)
-        return false;
-    const long groups = (ncols + C::CPB - 1) / C::CPB, cap = (long)sms * per;
+    static PerDevice<int> caps;
+    int &cap = caps.here();
+    if (!cap) {
+        if (cudaFuncSetAttribute(k_wavefieldsep<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM) != cudaSuccess)
+            return false;
+        int dev = 0, sms = 0, per = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_wavefieldsep<K>, C::NT, C::SMEM) != cudaSuccess || per < 1)
+            return false;
+        cap = sms * per;
+    }
+    const long groups = (ncols + C::CPB - 1) / C::CPB;
     k_wavefieldsep<K><<<(unsigned)(groups < cap ? groups : cap), C::NT, C::SMEM, s>>>(
         ncols, (int)g.nz, isfwi ? 1 : 0, F.v, F.b, F.pold, F.mold, dp, dm, dv);
     return true;
