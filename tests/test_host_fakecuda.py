@@ -127,3 +127,18 @@ for groups, per in {list(want)!r}:
     print(len(log("copy")), len(launches()))
 """)
     assert out == [f"{n} 1" for n in want.values()], out
+
+
+def test_run_allocates_scratch_only_for_steps_that_use_it():
+    """Grid-sized allocations of WFD_Prop_Run: none where one kernel does the step."""
+    want = {("Prop3DAcoIsoDenQ_DEO2_FDTD", 30, 20, 17): 0, ("Prop3DAcoIsoDenQ_DEO2_FDTD", 30, 20, 16): 0,
+            ("Prop3DAcoTTIDenQ_DEO2_FDTD", 30, 20, 16): 0, ("Prop3DAcoVTIDenQ_DEO2_FDTD", 30, 20, 17): 6,
+            ("Prop2DAcoIsoDenQ_DEO2_FDTD", 300, 0, 170): 3}
+    out = run(f"""
+for name, nx, ny, nz in {list(want)!r}:
+    a, p = create(name, nx, ny, nz)
+    fake.fake_reset()
+    rc = lib.WFD_Prop_Run(p, 5, 1, None, None, None, None, 5, 1)
+    print(rc, sum(int(n) >= 4 * nx * max(ny, 1) * nz for _, n in log("alloc")))
+""")
+    assert out == [f"0 {n}" for n in want.values()], out

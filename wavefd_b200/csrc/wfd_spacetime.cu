@@ -440,8 +440,9 @@ extern "C" int WFD_Prop_Run(void *prop, long nsteps, long it0, void *src_table, 
         return WFD_ERR_ARG;
     if (p->status) return p->status;
     cudaStream_t s = p->stream;
-    // scratch of the unfused passes must exist before a capture (no allocation inside a graph)
-    if (!p->fused || p->ndim == 2 || p->nz % 4 != 0)
+    // scratch of the unfused passes must exist before a capture (no allocation inside a graph); the fused 3D Iso step
+    // takes every grid
+    if (!p->fused || p->ndim == 2 || (p->nz % 4 != 0 && p->phys != wfd::ISO))
         if (!wfd::ensure_scratch(p, p->phys == wfd::ISO ? 3 : 6)) return p->status;
     const bool run2d = p->ndim == 2 && p->fused && !p->illum && nsteps > 0 && (!src || src->t.ngroups <= 1024);
     long *d_it = nullptr;
