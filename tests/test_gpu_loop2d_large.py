@@ -61,3 +61,25 @@ def test_source_points_beyond_the_grid_are_left_out(physics):
     got = _run(physics, shape, True, inside + [(nx * nz + 1, 1, 3.0), ((nx + 200) * nz + 8, 2, 5.0)], rec)
     for k in want:
         assert np.array_equal(got[k], want[k]), k
+
+
+# (nx, nz): tiles of 16 x 64 with 1, 11, 15 and 5 rows and 3, 2, 3, 9 and 63 columns over; row pairs that straddle the
+# last computed row and the grid's end (odd nx)
+SHAPES = [(5009, 67), (1211, 706), (4015, 131), (9509, 9), (1185, 575)]
+
+
+@pytest.mark.parametrize("physics", ["Iso", "VTI", "TTI"])
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("fs", [True, False])
+@pytest.mark.parametrize("acquisition", [True, False])
+def test_loop_is_the_stepping_calls_bit_for_bit(physics, shape, fs, acquisition):
+    nx, nz = shape
+    pt = lambda x, z, ir, c: (x * nz + z + 1, ir, c)  # noqa: E731
+    spts = [pt(nx // 2, nz // 2, 1, 1.0), pt(nx // 2, nz // 2, 2, 0.5), pt(nx - 1, nz - 1, 2, 0.25), pt(4, 4, 1, 0.3),
+            pt(nx - 5, nz - 5, 1, 0.7), pt(0, 0, 2, 0.1)]
+    rpts = [pt(x, min(3, nz - 1), x + 1, 1.0) for x in range(nx)] + [pt(nx // 2, nz // 2, 2, 0.5)]
+    if not acquisition:
+        spts = rpts = []
+    got, want = (_run(physics, shape, fs, spts, rpts, loop) for loop in (True, False))
+    for k in want:
+        assert np.isfinite(want[k]).all() and np.array_equal(got[k], want[k]), f"{physics} {shape} fs={fs} {k}"
