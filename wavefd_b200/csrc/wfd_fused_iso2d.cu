@@ -475,7 +475,7 @@ int iso2d_run(const Grid &g, const Fields &F, long nsteps, long it0, const RunEx
     };
     static PerDevice<Cap> caps;
     Cap &c = caps.here();
-    if (!c.known) {
+    if (!__atomic_load_n(&c.known, __ATOMIC_ACQUIRE)) {
         int dev = 0, sms = 0, per = 0, per_res = 0, coop = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
@@ -484,7 +484,9 @@ int iso2d_run(const Grid &g, const Fields &F, long nsteps, long it0, const RunEx
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_iso2d_run, NT, 0);
 #endif
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_res, k_iso2d_run_res, NT, 0);
-        c = Cap{true, coop ? sms * per : 0, coop ? sms * per_res : 0};
+        c.run = coop ? sms * per : 0;
+        c.res = coop ? sms * per_res : 0;
+        __atomic_store_n(&c.known, true, __ATOMIC_RELEASE);
     }
     const int cap = c.run, cap_res = c.res;
     const long ntiles = ((g.nz + TZ - 1) / TZ) * ((g.nx + TX - 1) / TX);

@@ -14,9 +14,8 @@
 // 2-3 quads per thread, sliding along z); then every thread applies D- and the time update to its
 // 4 cells and stores pOld and pSpace as float4.
 // The reference's region rules (interior [4,n-4), free-surface rows, untouched annulus) are
-// applied as selects on values computed everywhere; three code variants: interior tiles (no
-// selects), edge tiles (selects), and the top tile with a free surface (selects plus the image
-// stencils above kz = 0, which only the first z quad needs).
+// applied as selects on values computed everywhere, in one code path for all tiles; the image stencils
+// above a free surface's kz = 0 run for the first z quad of the top tile only.
 // Persistent CTAs loop over (tile, x-chunk) items; a chunk starts by filling its queues from global memory in
 // one go (all of its loads in flight together) and only then asks for its first groups. 14 warm-up planes
 // through the pipeline, each a wait for a whole group, took 5.1 us more a chunk, and so kept chunks above 16
@@ -56,8 +55,6 @@ constexpr int OFF_BAR = OFF_TZ + TY * TZW;
 constexpr size_t SMEM_BYTES = (size_t)OFF_BAR * 4 + NS * 8 + 16;
 static_assert(OFF_BAR % 2 == 0, "mbarrier alignment");
 static_assert((STAGE * 4) % 128 == 0 && (S_BH * 4) % 128 == 0 && (S_PN * 4) % 128 == 0, "TMA destination alignment");
-
-enum Mode { INNER = 0, EDGE = 1, TOP = 2 };
 
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 __device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
@@ -150,7 +147,6 @@ __device__ __forceinline__ unsigned ext_mask(const Grid &g, int tid, int z0, int
 }
 
 // pass-1 y/z outputs of the centre plane j into TYs/TZs (emask: ext_mask of this thread)
-template <int MODE>
 __device__ __forceinline__ void ext_stage(const Grid &g, const bool xin, const bool top, const int z0,
                                           const unsigned emask, const float *st, float *TYs, float *TZs) {
     const int tid = threadIdx.x;
@@ -176,7 +172,7 @@ __device__ __forceinline__ void ext_stage(const Grid &g, const bool xin, const b
                                       half2(w[rr + 3], h), half2(w[rr + 4], h), half2(w[rr + 5], h),
                                       half2(w[rr + 6], h), half2(w[rr + 7], h));
                 float2 t = mul2(half2(b, h), mul2(bc2(g.idy), s));
-                if (MODE != INNER) t = keep2(em, 4 * rr + 2 * h, t, zero);
+                t = keep2(em, 4 * rr + 2 * h, t, zero);
                 out[h] = t;
             }
             st4(TYs + r * TZ + 4 * zq, make_float4(out[0].x, out[0].y, out[1].x, out[1].y));
@@ -213,7 +209,7 @@ __device__ __forceinline__ void ext_stage(const Grid &g, const bool xin, const b
                     s = st8(g, pm(m - 3), pm(m - 2), pm(m - 1), pm(m), pm(m + 1), pm(m + 2), pm(m + 3), pm(m + 4));
                 }
                 float t = at(b, m) * (g.idz * s);
-                if (MODE != INNER) t = ((em >> (4 * k + m)) & 1u) ? t : 0.0f;
+                t = ((em >> (4 * k + m)) & 1u) ? t : 0.0f;
                 out[m] = t;
             }
             st4(TZs + r * TZW + 4 * qi, make_float4(out[0], out[1], out[2], out[3]));
@@ -223,7 +219,7 @@ __device__ __forceinline__ void ext_stage(const Grid &g, const bool xin, const b
 
 // D- in y and z, the time update and the stores of this thread's 4 cells (fmask bit m: the
 // reference updates cell m, given x)
-template <int MODE, bool EPI, bool RAG>
+template <bool EPI, bool RAG>
 __device__ __forceinline__ void fin_stage(const Grid &g, const long j, const bool xin, const bool top, const int z,
                                           const int y, const unsigned fmask, const int zq, const int row,
                                           const float2 *sx, const float2 *pc, float *st, const float *TYs,
@@ -280,11 +276,8 @@ __device__ __forceinline__ void fin_stage(const Grid &g, const long j, const boo
         const float2 k2 = div2(mul2(mul2(bc2(g.dt2), V), V), half2(b4, h));
         const float2 t = sub2(sub2(mul2(k2, L), mul2(half2(q4, h), sub2(pcv, pov))), pov);
         float2 np = add2(t, mul2(bc2(2.0f), pcv));
-        float2 nl = L;
-        if (MODE != INNER) {
-            np = keep2(fm, m0, np, pov);  // cells the reference leaves alone
-            nl = keep2(fm, m0, nl, bc2(0.0f));
-        }
+        np = keep2(fm, m0, np, pov);  // cells the reference leaves alone
+        float2 nl = keep2(fm, m0, L, bc2(0.0f));
         if (EPI && epi->scale_space)  // ScaleSpatialDerivatives fused (.h:269-291): pSpace *= V^2/B
             nl = mul2(nl, div2(mul2(V, V), half2(b4, h)));
         if (EPI && epi->born_dv) {
@@ -583,10 +576,10 @@ __global__ void __launch_bounds__(NT, 3)
             {
                 const bool xin = j >= 4 && j < g.nx - 4;
                 // one code path for every tile (the selects are cheap, code size is not)
-                ext_stage<EDGE>(g, xin, tile_top, z0, emask, st, TYs, TZs);
+                ext_stage(g, xin, tile_top, z0, emask, st, TYs, TZs);
                 __syncthreads();
-                if (own) fin_stage<EDGE, EPI, RAG>(g, j, xin, tile_top, z, y, fmask, zq, row, sx, pc, st, TYs, TZs, out_pold,
-                                               out_pspace, BATCH ? nullptr : F.illum, EPI ? &F.epi : nullptr, ea, eb);
+                if (own) fin_stage<EPI, RAG>(g, j, xin, tile_top, z, y, fmask, zq, row, sx, pc, st, TYs, TZs, out_pold,
+                                             out_pspace, BATCH ? nullptr : F.illum, EPI ? &F.epi : nullptr, ea, eb);
                 if (RAG) ragged_store(g, j, z0, y0, st, out_pold, out_pspace);
             }
             __syncthreads();

@@ -1,9 +1,10 @@
 // Unfused kernels: the reference's pass structure on the GPU, one thread per cell.
 //
 // These serve the Born-injection and imaging-condition entry points (which the reference
-// builds from standalone D+/D- passes and pointwise loops) and act as the unfused time step of 2D
-// and of small 3D grids (the larger ones: wfd_pass3d.cu) for geometries the fused kernels do not take. Per-cell arithmetic follows the reference's
-// expression trees; see the file:line notes at each kernel.
+// builds from standalone D+/D- passes and pointwise loops) and act as the unfused time step for
+// geometries the fused kernels do not take: 2D, and the 3D grids that are small or thin (pass3d_takes(); the
+// others: wfd_pass3d.cu). Per-cell arithmetic follows the reference's expression trees; see the file:line
+// notes at each kernel.
 #include "wfd_kernels.h"
 
 namespace WFD_NS {

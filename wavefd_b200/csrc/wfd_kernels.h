@@ -134,25 +134,15 @@ struct TileInfo {
                 float *oy, float *oz, cudaStream_t s);                                                   \
     bool fused_iso2d(const wfd::Grid &g, const wfd::Fields &F, cudaStream_t s);                          \
     bool fused_aniso2d(const wfd::Grid &g, int phys, int linear, const wfd::Fields &F, cudaStream_t s);  \
-    /* whole 2D Iso time loop in one cooperative launch: 0 launched, -1 not available, 1 launch error */ \
+    /* whole 2D Iso time loop in one cooperative launch: 0 launched, -1 not available, 1 launch error.  \
+       Fast build: only where every tile has its own co-resident CTA (else -1: loop2d_run) */           \
     int iso2d_run(const wfd::Grid &g, const wfd::Fields &F, long nsteps, long it0, const wfd::RunExtract &ex, \
                   unsigned *sync_words, cudaStream_t s);                                                 \
-    /* the same for 2D VTI and TTI (phys), the tiles shared out over the co-resident CTAs */           \
-    int aniso2d_run(const wfd::Grid &g, int phys, const wfd::Fields &F, long nsteps, long it0,          \
-                    const wfd::RunExtract &ex, unsigned *sync_words, cudaStream_t s);                    \
-    bool fused_iso2d(const wfd::Grid &g, const wfd::Fields &F, cudaStream_t s);                          \
-    bool fused_aniso2d(const wfd::Grid &g, int phys, int linear, const wfd::Fields &F, cudaStream_t s);  \
-    /* whole 2D Iso time loop in one cooperative launch: 0 launched, -1 not available, 1 launch error */ \
-    int iso2d_run(const wfd::Grid &g, const wfd::Fields &F, long nsteps, long it0, const wfd::RunExtract &ex, \
-                  unsigned *sync_words, cudaStream_t s);                                                 \
-    /* the same for 2D VTI and TTI (phys), the tiles shared out over the co-resident CTAs */           \
+    /* the same for 2D VTI and TTI (phys) */                                                            \
     int aniso2d_run(const wfd::Grid &g, int phys, const wfd::Fields &F, long nsteps, long it0,          \
                     const wfd::RunExtract &ex, unsigned *sync_words, cudaStream_t s);                    \
     /* 3D Iso: 0 not handled, 1 stepped (rows staged by cp.async: F.illum and F.epi not applied), 2    \
        stepped with F.illum and F.epi */                                                                 \
-    int fused_iso3d_tma(const wfd::Grid &g, const wfd::Fields &F, cudaStream_t s);                       \
-    /* 3D Iso: 0 not handled, 1 stepped (ragged rows: F.illum and F.epi not applied), 2 stepped with     \
-       F.illum and F.epi */                                                                              \
     int fused_iso3d_tma(const wfd::Grid &g, const wfd::Fields &F, cudaStream_t s);                       \
     /* a 2D loop as two passes a step with a barrier between (fast build only; S: 2 or 4 scratch arrays) */ \
     int loop2d_run(const wfd::Grid &g, int phys, const wfd::Fields &F, const wfd::Scratch &S, long nsteps, \

@@ -12,12 +12,13 @@
 // arithmetic. Global loads are single floats, coalesced along z; columns and rows outside the grid read
 // the nearest cell and are selected away.
 //
-// 60 (Iso), 116 (VTI) and 132 (TTI) bytes a cell in the two passes together, at half of HBM's rate: bound by
-// the latency of a plane's loads at 16 warps an SM. 203 x 181 x 251 a step: TTI 302 us, VTI 286 us (one
-// thread a cell with 64-bit index arithmetic, 428 instructions a cell and pass where these take 218:
+// 60 (Iso), 116 (VTI) and 132 (TTI) bytes a cell in the two passes together, TTI at 61 % of the measured 6547
+// GB/s: bound by the latency of a plane's loads at 16 warps an SM. 203 x 181 x 251 a step: TTI 302 us, VTI 286
+// us (one thread a cell with 64-bit index arithmetic, 428 instructions a cell and pass where these take 218:
 // 403 and 321 us). Tried and slower: 3 CTAs an SM (80 registers: fewer loads in flight, TTI 433 us); every
-// array through cp.async two planes ahead (LSU queues, TTI 317 us); 4 rows of CTAs of 128 threads (TTI
-// 290 us, but 10 % slower at 64^3). Chunks of 8, 16 and 32 planes: 305, 302, 336 us.
+// array through cp.async two planes ahead (LSU queues, TTI 317 us). Chunks of 8, 16 and 32 planes: 305, 302,
+// 336 us. CTAs of 128 threads took 290 us there (TTI; 10 % longer at 64^3, which these kernels are not given): not
+// taken up, other sizes were not measured.
 #include "wfd_kernels.h"
 
 namespace WFD_NS {

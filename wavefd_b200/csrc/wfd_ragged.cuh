@@ -5,7 +5,7 @@
 // its copies have landed. A warp takes whole rows: 32 columns at a time, then the columns beyond them
 // of several rows together. There are no bounds checks: a box that reaches past the grid's sides
 // reads whatever the flat address holds (a neighbouring row or plane, or the margin that
-// propagator arrays of such grids are allocated with on both ends, kRaggedMargin), because no cell
+// propagator arrays of such grids are allocated with on both ends, field_margin()), because no cell
 // that the reference computes uses a value from outside the grid and the kernels select, never
 // multiply, the other cells away. With per-copy bounds tests and zero fill the 3D Iso step took 282
 // us at 301 x 203 x 251, 180 us without.
