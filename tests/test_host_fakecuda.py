@@ -142,3 +142,17 @@ for name, nx, ny, nz in {list(want)!r}:
     print(rc, sum(int(n) >= 4 * nx * max(ny, 1) * nz for _, n in log("alloc")))
 """)
     assert out == [f"0 {n}" for n in want.values()], out
+
+
+def test_every_allocation_of_a_snapshot_file_is_checked(tmp_path):
+    code = f"""
+lib.WFD_Snap_Close.argtypes = [ctypes.c_void_p]
+before = fake.fake_live()
+f = lib.WFD_Snap_Open({str(tmp_path / "s")!r}.encode(), 3, 5000, 0)
+print("FILE" if f else "NULL", lib.WFD_LastError(), fake.fake_live() - before if not f else len(log("alloc")))
+if f: lib.WFD_Snap_Close(f)
+"""
+    kind, rc, n = run(code)[-1].split()
+    assert kind == "FILE" and int(n) >= 2
+    for k in range(1, int(n) + 1):
+        assert run(code, WAVEFD_B200_FAIL_ALLOC=str(k))[-1] == "NULL 2 0", k

@@ -386,7 +386,7 @@ extern "C" void *WFD_Snap_Open(const char *path, long nfields, long max_bytes, i
         cudaError_t e = cudaGetDevice(&f->device);
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&f->copy, cudaStreamNonBlocking);
         for (auto &s : f->stage) {
-            if (e == cudaSuccess) e = cudaHostAlloc(&s.host, (size_t)f->slot, cudaHostAllocDefault);
+            if (e == cudaSuccess) e = wfd::dMallocHost(&s.host, (size_t)f->slot);
             if (e == cudaSuccess) e = wfd::dMalloc(&s.dev, (size_t)f->slot);
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s.host_ev, cudaEventDisableTiming);
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s.dev_free_ev, cudaEventDisableTiming);
