@@ -382,8 +382,8 @@ __global__ void __launch_bounds__(NT, 1)
             float *s = sm + OFF_MAT + (gidx % NM) * M_STAGE;
             float *c = s + NMAT * MBOX;
             const int P = (int)(jstart + q + 3), j = (int)(jstart + q);
-            // The planes before the chunk only run pass 1: without pass 2's five boxes a step takes 1612 us at 400^3
-            // (1621 with them). Leaving out their halo outputs too was slower (1627: more registers, a branch).
+            // The planes before the chunk only run pass 1: without pass 2's five boxes a step alone takes 1614 us at
+            // 400^3 (1627 with them) and 458 at 256^3 (463); with several objects in turn the times are equal. Leaving out their halo outputs too was slower (1627: more registers, a branch).
             const bool core = q >= WARMUP;
             mbar_expect_tx(bar, 4u * (nmat * MBOX + (core ? NCORE * CBOX : 0)));
             tma_load_3d(s + MT_B * MBOX, mB, bar, z0 - 4, y0 - 4, P);

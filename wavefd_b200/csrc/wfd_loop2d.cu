@@ -8,8 +8,9 @@
 //
 // Two CTAs of 512 threads an SM; a warp's lanes are 32 z columns, a thread two consecutive x rows, whose
 // derivatives are formed as packed FP32 pairs; CTAs take turns over tiles of 64 z x 16 x cells (CTAs of 256,
-// 384 and 1024 threads and tiles 32 and 128 wide were within 10 %). Bound by L1 and L2: some 60 loads a
-// cell in Iso and VTI, 113 in TTI. Per step: pass 1 (the derivatives and the material sandwich) into scratch
+// 384 and 1024 threads and tiles 32 and 128 wide were within 10 %). Bound by the latency of the loads from L1 and
+// L2 at 32 warps an SM: some 60 loads a cell in Iso and VTI, 113 in TTI (2400 x 1200: long-scoreboard stalls 12 of
+// 21 per issue, l1tex 47 %, L2 20 %, DRAM 34 % busy). Per step: pass 1 (the derivatives and the material sandwich) into scratch
 // arrays, a grid-wide barrier (bounded, 1.3 us), pass 2 (the divergence and the update) with the step's
 // source injection, a barrier, the receivers. Everything stays in L2 up to about 2 M cells; stencil windows
 // are plain loads whose reuse within a CTA L1 serves (the barrier's acquire drops what other CTAs may have

@@ -29,7 +29,7 @@
 // tables in global memory, so calls on any streams and of any nz share nothing.
 //
 // Bound by shared-memory traffic and FP32 issue (about 90 kflop a column at nz = 300), not by the
-// 24 B/cell that have to move. A whole call (3D Iso, 160 x 128 x 300 cells, nz no power of two): 153 us;
+// 24 B/cell that have to move: l1tex 63 %, issue 51 % busy. A whole call (3D Iso, 160 x 128 x 300 cells, nz no power of two): 151 us;
 // one CTA a column with radix-2 stages and sincospif twiddles took 5580 us.
 #include "wfd_kernels.h"
 
