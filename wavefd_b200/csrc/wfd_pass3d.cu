@@ -364,8 +364,8 @@ int chunk_of(const Grid &g, dim3 &grid) {
 
 // Grids of a million cells and more whose tiles are well filled; the others take one thread a cell
 // (wfd_generic.cu). Smaller grids stay in L2 and are bound by the latency of a launch, which one thread a cell hides
-// better: TTI 80 x 75 x 69 21.2 us a step there and 23.0 here (100 x 110 x 90 41.6 and 36.9: the times cross below
-// the line, but between few cells and many the filling of the tiles moves the crossing more than the count).
+// better: TTI 80 x 75 x 69 (414,000 cells) 21.2 us a step there and 23.0 here. The times cross below the line (TTI 100 x
+// 110 x 90, 990,000 cells, 41.6 and 36.9); where between these two sizes was not measured, nor for VTI.
 // A tile costs the same however much of it is computed, so the second rule is on a plane's tile cells per computed
 // cell, r. us a step there and here, on both sides of each line: VTI (r <= 1.32) 250 x 90 x 90 r 1.31 78.9, 74.7;
 // 160 x 140 x 101 r 1.44 88.6, 88.2; 300 x 300 x 50 r 1.45 172, 182; 12000 x 9 x 10 r 85 33.9, 131.5. TTI (1.6)
