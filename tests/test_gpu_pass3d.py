@@ -39,3 +39,28 @@ def test_marching_step(oracle, physics, shape, fs, linear):
             a, b = gpu.arr(k), orc.arr(k)
             assert same(a, b) if strict else rel_l2(a, b) <= 1e-5, f"{name} {shape} strict={strict} {k}"
         gpu.close()
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("fs", [True, False])
+def test_marching_step_iso_unfused(oracle, shape, fs):
+    """3D Iso takes the two passes with the fused kernels off (WFD_Prop_SetFused)."""
+    from wavefd_b200 import _lib
+    lib, name = _lib.library(), "Prop3DAcoIsoDenQ_DEO2_FDTD"
+    model = make_model(3, "iso", shape, seed=3)
+    orc = OracleRunner(oracle, name, shape, fs=fs)
+    orc.load(model)
+    for _ in range(4):
+        orc.step()
+    for strict in (1, 0):
+        gpu = ABIRunner(lib, name, shape, fs=fs)
+        lib.WFD_Prop_SetStrict(ctypes.c_void_p(gpu.p), strict)
+        lib.WFD_Prop_SetFused(ctypes.c_void_p(gpu.p), 0)
+        gpu.load(model)
+        for _ in range(4):
+            gpu.abi.TimeStep(gpu.p)
+        assert lib.WFD_Prop_Status(ctypes.c_void_p(gpu.p)) == 0 and lib.WFD_Prop_StepKernels(ctypes.c_void_p(gpu.p)) == 2
+        for k in ("PCur", "POld", "PSpace"):
+            a, b = gpu.arr(k), orc.arr(k)
+            assert same(a, b) if strict else rel_l2(a, b) <= 1e-5, f"{shape} strict={strict} {k}"
+        gpu.close()
