@@ -94,7 +94,7 @@ def test_two_pass_kernels_by_size(physics):
     from tests.test_gpu_pass3d import SHAPES
     marching = [(nx, ny, nz) for nz, ny, nx in SHAPES] + [(203, 181, 251), (250, 90, 90), (16, 400, 301), (80, 112, 126)]
     cells = [(12000, 9, 10), (3000, 17, 33), (2000, 33, 17), (20, 20, 3001), (40, 33, 1001), (300, 18, 301), (300, 300, 33),
-             (600, 33, 65), (9, 1000, 301), (101, 100, 101), (64, 60, 67)]
+             (600, 33, 65), (300, 70, 70), (64, 60, 67)]
     for line in _two_pass(physics, marching):
         assert "k_pass1_3d" in line and "k_pass2_3d" in line, line
     for size, line in zip(cells, _two_pass(physics, cells)):
@@ -103,7 +103,7 @@ def test_two_pass_kernels_by_size(physics):
 
 def test_two_pass_kernels_between_the_lines():
     """Where only one physics gains."""
-    sizes = [(400, 180, 50), (300, 300, 50), (150, 113, 135)]
+    sizes = [(400, 180, 50), (101, 100, 101), (200, 97, 97), (9, 1000, 301)]
     assert all("_3d" not in line for line in _two_pass("VTI", sizes))
     assert all("k_pass1_3d" in line for line in _two_pass("TTI", sizes))
 

@@ -367,18 +367,22 @@ int chunk_of(const Grid &g, dim3 &grid) {
 // better: TTI 80 x 75 x 69 (414,000 cells) 21.2 us a step there and 23.0 here. The times cross below the line (TTI 100 x
 // 110 x 90, 990,000 cells, 41.6 and 36.9); where between these two sizes was not measured, nor for VTI.
 // A tile costs the same however much of it is computed, so the second rule is on a plane's tile cells per computed
-// cell, r. us a step there and here, on both sides of each line: VTI (r <= 1.32) 250 x 90 x 90 r 1.31 78.9, 74.7;
-// 160 x 140 x 101 r 1.44 88.6, 88.2; 300 x 300 x 50 r 1.45 172, 182; 12000 x 9 x 10 r 85 33.9, 131.5. TTI (1.6)
-// 400 x 180 x 50 r 1.55 172.8, 162.9; 101 x 100 x 101 r 1.61 46.0, 47.4; 300 x 70 x 70 r 1.88 67.7, 72.4; Iso (1.5)
-// 150 x 113 x 136 r 1.48 50.4, 45.9; 300 x 300 x 44 r 1.67 90.8, 99.6. Below 12 planes the zeros that each CTA
-// writes on the planes beside the computed ones show: VTI 9 x 1000 x 301 36.5, 41.3; 14 x 310 x 319 32.4, 31.7.
+// cell, r. The lines lie between those of one object stepping alone and of several in turn, whose launches fill each
+// other's last waves; us a step there and here, alone; in turn, on both sides of each line:
+//   VTI (r <= 1.5)   150 x 113 x 135 r 1.49 88.6, 90.0; 77.5, 77.6    300 x 300 x 50 r 1.45 172, 182; 160, 146
+//                    101 x 100 x 101 r 1.61 39.8, 42.4; 35.2, 38.7    12000 x 9 x 10 r 85 33.9, 131.5 (alone)
+//   TTI (r <= 1.85)  200 x 120 x 67 r 1.74 72.2, 65.7 (in turn)       101 x 100 x 101 r 1.61 46.0, 47.4; 44.4, 41.3
+//                    300 x 70 x 70 r 1.88 67.7, 72.4; 64.6, 62.3      300 x 22 x 301 r 2.46 77.3, 95.9; 69.9, 82.0
+//   Iso (r <= 1.5)   150 x 113 x 136 r 1.48 50.4, 45.9 (alone)        300 x 300 x 44 r 1.67 90.8, 99.6 (alone)
+// Below 12 planes the zeros that each CTA writes on the planes beside the computed ones show, in TTI less than the
+// gain: VTI 9 x 1000 x 301 36.5, 41.3; 35.2, 38.2, TTI 43.8, 42.3; 41.7, 39.0; VTI 14 x 310 x 319 32.4, 31.7; 31.6, 27.7.
 bool pass3d_takes(const Grid &g, int phys) {
-    if (g.ndim != 3 || g.n < 1000000 || g.nx < 12) return false;
+    if (g.ndim != 3 || g.n < 1000000 || (phys != TTI && g.nx < 12)) return false;
     const long nty = (g.ny + TY - 1) / TY, ntz = (g.nz + TZ - 1) / TZ;
     if (nty > 65535 || ntz >= 2147483647L) return false;
     const double staged = (double)(ntz * TZ) * (double)(nty * TY);
     const double computed = (double)(g.ny - 8) * (double)(g.nz - (g.fs ? 4 : 8));
-    return staged <= (phys == TTI ? 1.6 : (phys == VTI ? 1.32 : 1.5)) * computed;
+    return staged <= (phys == TTI ? 1.85 : 1.5) * computed;
 }
 
 void pass1_3d(const Grid &g, int phys, const Fields &F, const Scratch &S, cudaStream_t s) {
